@@ -410,6 +410,7 @@ int tdgl_snapshot_restore(tdgl_ctx *c, int32_t slot) {
   int rc = snap_copy(ctx, sn, false);
   if (rc) return rc;
   ctx->steps = sn.steps;
+  ctx->outside_state = true;
   if (ctx->pcg) pcg_flags(ctx, &sn.warm, &sn.have2, true);
   if (ctx->open) *open_count_ptr(ctx) = sn.open_count;
   return 0;
@@ -663,6 +664,7 @@ int tdgl_upload_state(tdgl_ctx *c, const tdgl_state_view *s) {
   }
   TDGL_CUDA(cudaStreamSynchronize(ctx->stream));
   ctx->have_state = true;
+  ctx->outside_state = true;
   return 0;
 }
 
@@ -727,6 +729,13 @@ static int ss_reserve(Ctx *ctx, int n) {
   return 0;
 }
 
+// what the first step on a state from outside (an upload, a snapshot) does once, before the step
+static void state_came_in(Ctx *ctx) {
+  if (!ctx->outside_state) return;
+  clear_outside(ctx);
+  ctx->outside_state = false;
+}
+
 static int deferred_status(Ctx *ctx) {
   const int st = ctx->P.solver == TDGL_SOLVER_PCG ? pcg_take_status(ctx) : 0;
   if (st == TDGL_ENOCONV) set_err(ctx, st, "PCG reached maxit without meeting its tolerance");
@@ -740,6 +749,7 @@ static int run_steps(Ctx *ctx, int32_t n, double H, const double *HJs, double HJ
   ctx->launches = 0;
   int rc = ss_reserve(ctx, n);
   if (rc) return rc;
+  if (n > 0) state_came_in(ctx);
   const bool open = ctx->P.selffield_bc == TDGL_BC_OPEN;
   for (int q = 0; q < n; q++) {
     const double hj = HJs ? HJs[q] : HJ;
@@ -1141,6 +1151,7 @@ static int batch_launch(tdgl_batch_impl *b, int m, const double *H, const double
     const bool open = ctx->P.selffield_bc == TDGL_BC_OPEN;
     any_open = any_open || open;
     if ((rc = ss_reserve(ctx, open ? m : 1))) return rc;
+    if (m > 0) state_came_in(ctx);
     ctx->ss_last_ok = false;   // the batch graph advances the noise index on the device
     ctx->launches = 0;
     if (open) {

@@ -3,35 +3,40 @@
 // One kernel per band stage: the gauge-link stencil of _band_row! (bands.jl:71-97) with the KWT update
 // (kwt_update :135-140, kwt_update_rot :151-159), fused with the per-node epilogues that follow it in the
 // reference — the rotating-frame rate or term (_frame_rate! :213-234, _frame_term! :274-286), the RKL/RKC
-// combination (_combine! :425-430) and the final turn back (_frame_turn! :321-327).  Link rotations of the
-// later stages (_rot!, _advance_links!, _frame_links!, _link_rate!, _rotlinks!, _rotfrac!, :292-423) run as one
-// kernel over the three link ranges; the covariant Neumann ghosts (ghosts! :524-539) as three face passes in the
-// reference's precedence x, y, z.
+// combination (_combine! :425-430) and the final turn back (_frame_turn! :321-327).  The links of later RKL/RKC stages
+// (_rotlinks!, _rotfrac!) are formed where a stage reads them; the other link rotations (_rot!, _advance_links!,
+// _frame_links!, _link_rate!, :292-423) run as one kernel over the three link ranges.  The covariant Neumann ghosts of
+// an intermediate stage (ghosts! :524-539) are formed in the next stage too, the step's final ones by one pass over the
+// block's shell.
 #include "common.cuh"
 #include "merge.cuh"
 
 namespace tdgl {
 
-// The links a stage reads: the arrays as given (mode 0), or (mode 1) the rotated links of a later RKL/RKC stage of a
-// rotating-frame band, V e^{iRc} with the per-step rate R (_rotlinks!, bands.jl:311-316), formed on the fly from the
-// step's links where the stencil or the ghosts read them instead of from a stored copy: the same per-link formula as
-// the link pass.  (_rotfrac! of a band without the frame keeps its link pass.)
+// The links a stage reads: the arrays as given (mode 0), or the rotated links of a later RKL/RKC stage formed from the
+// step's links where the stencil reads them: (mode 1) V e^{iRc} with the per-step rate R of a rotating-frame band
+// (_rotlinks!, bands.jl:311-316), (mode 2) V Q^c with Q = V conj(U) of a band without the frame (_rotfrac!, :409-423).
+// The formulas are the link passes'.  Mode 2 replaces a pass per stage that read V and U and stored the result (144
+// bytes a node, and a launch) by 48 more bytes a node in the stage.
 struct LinkRot {
   int mode;
   double c;
   const cd *V[3], *U[3];
   const double *R[3];
 };
+__device__ __forceinline__ cd link_frac(cd v, cd u, double c);
 // LR: the mode, fixed per kernel instance
 template <int LR>
 __device__ __forceinline__ cd link_at(const LinkRot &R, const cd *L, int ax, long long o) {
   if (LR == 0) return L[o];
+  if (LR == 2) return link_frac(R.V[ax][o], R.U[ax][o], R.c);
   return cmul(R.V[ax][o], ccis_short(R.R[ax][o] * R.c));
 }
 
 struct StageArgs {
   cd *C;              // destination
   const cd *S;        // stage source
+  int gfly;           // 1: S is an intermediate stage, whose ghosts are formed here (see nbp / nbm)
   BandPtrs G;         // every band at the start of the step (coupling)
   const cd *Lx, *Ly, *Lz;
   const double *f;
@@ -114,6 +119,10 @@ TDGL_STAGE_MERGE(false, false, 1);
 TDGL_STAGE_MERGE(true, false, 1);
 TDGL_STAGE_MERGE(false, true, 1);
 TDGL_STAGE_MERGE(true, true, 1);
+TDGL_STAGE_MERGE(false, false, 2);
+TDGL_STAGE_MERGE(true, false, 2);
+TDGL_STAGE_MERGE(false, true, 2);
+TDGL_STAGE_MERGE(true, true, 2);
 template <bool MAT, bool VAC, int LR>
 __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
   long long t = (long long)bk.x * blockDim.x + threadIdx.x;
@@ -128,6 +137,22 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
   auto LZ = [&](long long q) { return link_at<LR>(A.lr, A.Lz, 2, q); };
   cd g = A.S[o];
   double fm = A.f[o];
+  // the stage source at the next (nbp) and previous (nbm) node along an axis.  A node beside a face reads its ghost:
+  // of an intermediate stage (gfly) the value ghosts! would have stored, L S of the node inside (which is this node) on
+  // the low face and conj(L) S on the high one, with this stage's own links (the same product, the same bits).  The
+  // stencil reads face points only, never edges.  This saves the ghost pass of every intermediate stage, a launch
+  // between two stages that cannot overlap it.  With the links of mode 2, the clamped Ω faces and no copy at the end,
+  // 40 steps went from 3318 to 2811 µs (12×8×4 cells), 4183 to 3782 (64×32×8), 8289 to 7893 (192×64×16), 10207 to
+  // 6841 (101×37×9 with noise) and 252.9 to 250.0 ms (the 256×128×32 ramp).
+  const Rng &rg = A.r;
+  auto nbp = [&](int ax, long long s, cd l) {
+    const bool edge = ax == 0 ? i == rg.i0 + rg.ni - 1 : ax == 1 ? j == rg.j0 + rg.nj - 1 : k == rg.k0 + rg.nk - 1;
+    return A.gfly && edge ? cmul(cconj(l), g) : A.S[o + s];
+  };
+  auto nbm = [&](int ax, long long s, cd lc) {   // lc: the conjugate of the previous link
+    const bool edge = ax == 0 ? i == rg.i0 : ax == 1 ? j == rg.j0 : k == rg.k0;
+    return A.gfly && edge ? cmul(cconj(lc), g) : A.S[o - s];
+  };
   cd v;
   if ((VAC && A.vac[o]) || (A.hard && fm == 0.0)) {
     v = mkc(0.0, 0.0);
@@ -145,9 +170,10 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
       wzp *= W[2][m][A.mat[o + sz] - 1];
       wzm *= W[2][A.mat[o - sz] - 1][m];
     }
-    cd tx = rmul(cf.kx, cadd(rmul(wxp, csub(cmul(LX(o), A.S[o + sx]), g)), rmul(wxm, csub(cmul(cconj(LX(o - sx)), A.S[o - sx]), g))));
-    cd ty = rmul(cf.ky, cadd(rmul(wyp, csub(cmul(LY(o), A.S[o + sy]), g)), rmul(wym, csub(cmul(cconj(LY(o - sy)), A.S[o - sy]), g))));
-    cd tz = rmul(cf.kz, cadd(rmul(wzp, csub(cmul(LZ(o), A.S[o + sz]), g)), rmul(wzm, csub(cmul(cconj(LZ(o - sz)), A.S[o - sz]), g))));
+    const cd lxp = LX(o), lxm = cconj(LX(o - sx)), lyp = LY(o), lym = cconj(LY(o - sy)), lzp = LZ(o), lzm = cconj(LZ(o - sz));
+    cd tx = rmul(cf.kx, cadd(rmul(wxp, csub(cmul(lxp, nbp(0, sx, lxp)), g)), rmul(wxm, csub(cmul(lxm, nbm(0, sx, lxm)), g))));
+    cd ty = rmul(cf.ky, cadd(rmul(wyp, csub(cmul(lyp, nbp(1, sy, lyp)), g)), rmul(wym, csub(cmul(lym, nbm(1, sy, lym)), g))));
+    cd tz = rmul(cf.kz, cadd(rmul(wzp, csub(cmul(lzp, nbp(2, sz, lzp)), g)), rmul(wzm, csub(cmul(lzm, nbm(2, sz, lzm)), g))));
     cd acc = cadd(cadd(cadd(cadd(g, tx), ty), tz), mulr(rmul(cf.c, g), fm * cf.eps - cf.beta * cabs2(g)));
     for (int nu = 0; nu < A.N; nu++) {
       if (nu == mu) continue;
@@ -162,13 +188,15 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
     const double(*W)[TDGL_MAXMAT][TDGL_MAXMAT] = A.mt->W[mu];
     const int mxp = A.mat[o + sx] - 1, mxm = A.mat[o - sx] - 1, myp = A.mat[o + sy] - 1, mym = A.mat[o - sy] - 1,
               mzp = A.mat[o + sz] - 1, mzm = A.mat[o - sz] - 1;
-    cd vxm = cconj(LX(o - sx)), vym = cconj(LY(o - sy)), vzm = cconj(LZ(o - sz));
-    cd tx = dif_mat(A.tau[0][o] * W[0][m][mxp], A.tau[0][o - sx] * W[0][mxm][m], cf.kx, LX(o), A.S[o + sx], vxm,
-                    A.S[o - sx], g);
-    cd ty = dif_mat(A.tau[1][o] * W[1][m][myp], A.tau[1][o - sy] * W[1][mym][m], cf.ky, LY(o), A.S[o + sy], vym,
-                    A.S[o - sy], g);
-    cd tz = dif_mat(A.tau[2][o] * W[2][m][mzp], A.tau[2][o - sz] * W[2][mzm][m], cf.kz, LZ(o), A.S[o + sz], vzm,
-                    A.S[o - sz], g);
+    const cd vxp = LX(o), vxm = cconj(LX(o - sx));
+    cd tx = dif_mat(A.tau[0][o] * W[0][m][mxp], A.tau[0][o - sx] * W[0][mxm][m], cf.kx, vxp, nbp(0, sx, vxp), vxm,
+                    nbm(0, sx, vxm), g);
+    const cd vyp = LY(o), vym = cconj(LY(o - sy));
+    cd ty = dif_mat(A.tau[1][o] * W[1][m][myp], A.tau[1][o - sy] * W[1][mym][m], cf.ky, vyp, nbp(1, sy, vyp), vym,
+                    nbm(1, sy, vym), g);
+    const cd vzp = LZ(o), vzm = cconj(LZ(o - sz));
+    cd tz = dif_mat(A.tau[2][o] * W[2][m][mzp], A.tau[2][o - sz] * W[2][mzm][m], cf.kz, vzp, nbp(2, sz, vzp), vzm,
+                    nbm(2, sz, vzm), g);
     const double eps = A.Th ? A.mt->a[mu][m] - A.Th[o] : cf.eps;   // _anode: the material's a (bands.jl:65-66)
     cd nl = mulr(rmul(cf.c, g), fm * eps - cf.beta * cabs2(g));
     cd acc = cadd(cadd(cadd(cadd(g, tx), ty), tz), nl);
@@ -181,11 +209,13 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
     if (A.mt->absent[mu][m]) v = mkc(0.0, 0.0);
   } else {
     const tdgl_bandcoef &cf = A.cf;
-    cd vxm = cconj(LX(o - sx)), vym = cconj(LY(o - sy)), vzm = cconj(LZ(o - sz));
     cd g2 = rmul(2.0, g);
-    cd tx = rmul(cf.kx, cadd(csub(cmul(LX(o), A.S[o + sx]), g2), cmul(vxm, A.S[o - sx])));
-    cd ty = rmul(cf.ky, cadd(csub(cmul(LY(o), A.S[o + sy]), g2), cmul(vym, A.S[o - sy])));
-    cd tz = rmul(cf.kz, cadd(csub(cmul(LZ(o), A.S[o + sz]), g2), cmul(vzm, A.S[o - sz])));
+    const cd vxp = LX(o), vxm = cconj(LX(o - sx));
+    cd tx = rmul(cf.kx, cadd(csub(cmul(vxp, nbp(0, sx, vxp)), g2), cmul(vxm, nbm(0, sx, vxm))));
+    const cd vyp = LY(o), vym = cconj(LY(o - sy));
+    cd ty = rmul(cf.ky, cadd(csub(cmul(vyp, nbp(1, sy, vyp)), g2), cmul(vym, nbm(1, sy, vym))));
+    const cd vzp = LZ(o), vzm = cconj(LZ(o - sz));
+    cd tz = rmul(cf.kz, cadd(csub(cmul(vzp, nbp(2, sz, vzp)), g2), cmul(vzm, nbm(2, sz, vzm))));
     const double eps = A.Th ? A.heat_a - A.Th[o] : cf.eps;
     cd nl = mulr(rmul(cf.c, g), fm * eps - cf.beta * cabs2(g));
     cd acc = cadd(cadd(cadd(cadd(g, tx), ty), tz), nl);
@@ -200,9 +230,9 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
         const double cx = c3[0] / A.ddiv, cy = c3[1] / A.ddiv, cz = c3[2] / A.ddiv;
         const cd *P = A.G.p[nu];
         const cd p2 = rmul(2.0, P[o]);
-        const cd ex = rmul(cx, cadd(csub(cmul(LX(o), P[o + sx]), p2), cmul(vxm, P[o - sx])));
-        const cd ey = rmul(cy, cadd(csub(cmul(LY(o), P[o + sy]), p2), cmul(vym, P[o - sy])));
-        const cd ez = rmul(cz, cadd(csub(cmul(LZ(o), P[o + sz]), p2), cmul(vzm, P[o - sz])));
+        const cd ex = rmul(cx, cadd(csub(cmul(vxp, P[o + sx]), p2), cmul(vxm, P[o - sx])));
+        const cd ey = rmul(cy, cadd(csub(cmul(vyp, P[o + sy]), p2), cmul(vym, P[o - sy])));
+        const cd ez = rmul(cz, cadd(csub(cmul(vzp, P[o + sz]), p2), cmul(vzm, P[o - sz])));
         acc = cadd(acc, cadd(cadd(ex, ey), ez));
       }
     if (cf.gamma2 > 0) v = A.rk ? kwt_update_rot(g, csub(acc, g), cf.gamma2) : kwt_update(g, csub(acc, g), cf.gamma2);
@@ -225,39 +255,16 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
   A.C[o] = v;
 }
 
-// Ω on the six faces of the block copies the node inside (bands.jl:224-232), one pass per axis.
-__device__ __forceinline__ void omega_face_b(const Blk bk, double * const &Om, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi);
-__global__ void k_omega_face(double *Om, Dim d, Rng r, int axis, int lo, int hi) { omega_face_b(TDGL_BLK, Om, d, r, axis, lo, hi); }
-TDGL_MERGEABLE(k_omega_face, omega_face_b, 256, 1, false);
-__device__ __forceinline__ void omega_face_b(const Blk bk, double * const &Om, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi) {
-  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
-  if (t >= r.n()) return;
-  int a, b, c;
-  rng_ijk(r, t, a, b, c);
-  if (axis == 0) {
-    Om[d.at(lo, b, c)] = Om[d.at(lo + 1, b, c)];
-    Om[d.at(hi + 1, b, c)] = Om[d.at(hi, b, c)];
-  } else if (axis == 1) {
-    Om[d.at(a, lo, c)] = Om[d.at(a, lo + 1, c)];
-    Om[d.at(a, hi + 1, c)] = Om[d.at(a, hi, c)];
-  } else {
-    Om[d.at(a, b, lo)] = Om[d.at(a, b, lo + 1)];
-    Om[d.at(a, b, hi + 1)] = Om[d.at(a, b, hi)];
-  }
-}
-
 // Covariant Neumann ghosts of one band on one pair of faces (bands.jl:524-539).
-__device__ __forceinline__ void ghost_face_b(const Blk bk, cd * const &X, const cd * const &Lk, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi, LinkRot const &lr);
-__global__ void k_ghost_face(cd *X, const cd *Lk, Dim d, Rng r, int axis, int lo, int hi, LinkRot lr) { ghost_face_b(TDGL_BLK, X, Lk, d, r, axis, lo, hi, lr); }
+__device__ __forceinline__ void ghost_face_b(const Blk bk, cd * const &X, const cd * const &Lk, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi);
+__global__ void k_ghost_face(cd *X, const cd *Lk, Dim d, Rng r, int axis, int lo, int hi) { ghost_face_b(TDGL_BLK, X, Lk, d, r, axis, lo, hi); }
 TDGL_MERGEABLE(k_ghost_face, ghost_face_b, 256, 1, false);
-__device__ __forceinline__ void ghost_face_b(const Blk bk, cd * const &X, const cd * const &Lk, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi, LinkRot const &lr) {
+__device__ __forceinline__ void ghost_face_b(const Blk bk, cd * const &X, const cd * const &Lk, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi) {
   long long t = (long long)bk.x * blockDim.x + threadIdx.x;
   if (t >= r.n()) return;
   int a, b, c;
   rng_ijk(r, t, a, b, c);
-  auto L = [&](long long q) {
-    return lr.mode == 0 ? link_at<0>(lr, Lk, axis, q) : link_at<1>(lr, Lk, axis, q);
-  };
+  auto L = [&](long long q) { return Lk[q]; };
   if (axis == 0) {
     X[d.at(lo, b, c)] = cmul(L(d.at(lo, b, c)), X[d.at(lo + 1, b, c)]);
     X[d.at(hi + 1, b, c)] = cmul(cconj(L(d.at(hi, b, c))), X[d.at(hi, b, c)]);
@@ -282,7 +289,6 @@ struct ShellArgs {
   long long nz_face, ny_face;   // points of the two z faces; of the two y faces (k inside)
   long long n;                  // all shell points
   Dim d;
-  LinkRot lr;                   // how Lx, Ly, Lz are read
 };
 
 __device__ __forceinline__ void ghost_shell_b(const Blk bk, ShellArgs const &A);
@@ -295,9 +301,7 @@ __device__ __forceinline__ void ghost_shell_b(const Blk bk, ShellArgs const &A) 
   const int x1 = A.x1, x2 = A.x2, y1 = A.y1, y2 = A.y2, z1 = A.z1, z2 = A.z2;
   const int ni = x2 - x1 + 2, nj = y2 - y1 + 2, nk = z2 - z1;   // the block's nodes per axis; inside k
   const cd *X = A.X;
-  auto lk = [&](const cd *L, int ax, long long q) {
-    return A.lr.mode == 0 ? L[q] : link_at<1>(A.lr, L, ax, q);
-  };
+  auto lk = [&](const cd *L, int, long long q) { return L[q]; };
   // the value each pass writes at (i, j, k), from the values before it
   auto vx = [&](int i, int j, int k) -> cd {   // x pass (reads the inside column)
     return i == x1 ? cmul(lk(A.Lx, 0, d.at(x1, j, k)), X[d.at(x1 + 1, j, k)]) : cmul(cconj(lk(A.Lx, 0, d.at(x2, j, k))), X[d.at(x2, j, k)]);
@@ -333,7 +337,7 @@ __device__ __forceinline__ void ghost_shell_b(const Blk bk, ShellArgs const &A) 
 }
 
 // Link operations over the three link ranges of the band stencil (_rx, _ry, _rz, bands.jl:349-351).
-enum LinkOp { LOP_ROT_INIT = 0, LOP_ADVANCE, LOP_FRAME_LINKS, LOP_LINK_RATE, LOP_ROTLINKS, LOP_ROTFRAC };
+enum LinkOp { LOP_ROT_INIT = 0, LOP_ADVANCE, LOP_FRAME_LINKS, LOP_LINK_RATE };
 
 struct LinkArgs {
   int op;
@@ -343,7 +347,8 @@ struct LinkArgs {
   const cd *V[3], *U[3];
   double *Rr[3];
   const double *Om;
-  double par;   // n (ROT_INIT), τ (FRAME_LINKS), dt (LINK_RATE), c (ROTLINKS / ROTFRAC)
+  Rng ri;       // the interior nodes, where Ω is stored
+  double par;   // n (ROT_INIT), τ (FRAME_LINKS), dt (LINK_RATE)
 };
 
 // The per-link formulas (bands.jl:303-310 _link_rate!, :355-369 _rot!, :409-423 _rotfrac!), shared by the step's
@@ -396,6 +401,10 @@ __device__ __forceinline__ void link_op_b(const Blk bk, LinkArgs const &A) {
   rng_ijk(A.r[ax], t, i, j, k);
   const long long o = A.d.at(i, j, k);
   const int oi = ax == 0, oj = ax == 1, ok = ax == 2;
+  // Ω along the link; a face point has the node inside (bands.jl:224-232: the copies x, then y, then z clamp each index)
+  auto dOm = [&]() {
+    return A.Om[om_at(A.d, A.ri, i + oi, j + oj, k + ok)] - A.Om[om_at(A.d, A.ri, i, j, k)];
+  };
   switch (A.op) {
     case LOP_ROT_INIT: {
       const cd v = A.V[ax][o];
@@ -407,26 +416,20 @@ __device__ __forceinline__ void link_op_b(const Blk bk, LinkArgs const &A) {
       A.L[ax][o] = cmul(A.L[ax][o], A.Rl[ax][o]);
       break;
     case LOP_FRAME_LINKS:
-      A.L[ax][o] = cmul(A.L[ax][o], ccis_short((A.Om[A.d.at(i + oi, j + oj, k + ok)] - A.Om[o]) * A.par));
+      A.L[ax][o] = cmul(A.L[ax][o], ccis_short(dOm() * A.par));
       break;
     case LOP_LINK_RATE:
-      A.Rr[ax][o] = link_angle(A.V[ax][o], A.U[ax][o]) + (A.Om[A.d.at(i + oi, j + oj, k + ok)] - A.Om[o]) * A.par;
-      break;
-    case LOP_ROTLINKS:
-      A.L[ax][o] = cmul(A.V[ax][o], ccis_short(A.Rr[ax][o] * A.par));
-      break;
-    case LOP_ROTFRAC:
-      A.L[ax][o] = link_frac(A.V[ax][o], A.U[ax][o], A.par);
+      A.Rr[ax][o] = link_angle(A.V[ax][o], A.U[ax][o]) + dOm() * A.par;
       break;
   }
 }
 
-__device__ __forceinline__ void copy_c_b(const Blk bk, cd * const &dst, const cd * const &src, long long const &n);
-__global__ void k_copy_c(cd *dst, const cd *src, long long n) { copy_c_b(TDGL_BLK, dst, src, n); }
-TDGL_MERGEABLE(k_copy_c, copy_c_b, 256, 1, false);
-__device__ __forceinline__ void copy_c_b(const Blk bk, cd * const &dst, const cd * const &src, long long const &n) {
-  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
-  if (t < n) dst[t] = src[t];
+// X = 0 on the nodes outside the block (x1..x2+1 and so on)
+__global__ void k_zero_outside(cd *X, Geo g) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= g.d.n()) return;
+  const int i = 1 + (int)(t % g.d.n1), j = 1 + (int)((t / g.d.n1) % g.d.n2), k = 1 + (int)(t / ((long long)g.d.n1 * g.d.n2));
+  if (i < g.x1 || i > g.x2 + 1 || j < g.y1 || j > g.y2 + 1 || k < g.z1 || k > g.z2 + 1) X[t] = mkc(0.0, 0.0);
 }
 
 namespace {
@@ -447,9 +450,10 @@ void link_op(Ctx *ctx, int op, double par) {
     A.L[ax] = ctx->L[ax]; A.Rl[ax] = ctx->Rl[ax]; A.V[ax] = ctx->V[ax]; A.U[ax] = ctx->U[ax]; A.Rr[ax] = ctx->Rr[ax];
   }
   A.Om = ctx->Om;
+  A.ri = interior(g);
   A.par = par;
   long long n = A.r[0].n() + A.r[1].n() + A.r[2].n();
-  static const double per[6] = {64, 48, 40, 48, 40, 48};   // compulsory bytes per link of each operation
+  static const double per[4] = {64, 48, 40, 48};   // compulsory bytes per link of each operation
   TDGL_LAUNCH(ctx, K_LINK, per[op] * n, k_link_op, nblk(n, BS), BS, 0, A);
 }
 
@@ -484,6 +488,7 @@ StageArgs stage_base(Ctx *ctx, int mu, const tdgl_bandcoef &cf, double ddiv) {
 double stage_bytes(const StageArgs &A) {
   double b = 16 + 16 + 8 + 48 + 16.0 * (A.N - 1);
   if (A.lr.mode == 1) b += 24;   // the rate R beside the links V
+  if (A.lr.mode == 2) b += 48;   // the links U of the step before
   if (A.combine) b += 16;
   if (A.frame_rate || A.frame_term || A.turn) b += 8;
   if (A.mat || A.vac) b += 24 + 1;   // τ along the three axes, the node's material or vacuum flag
@@ -501,7 +506,8 @@ void launch_stage(Ctx *ctx, const StageArgs &A) {
     else if (A.mat) TDGL_LAUNCH(ctx, K_BAND, by, (k_band_stage<true, false, LR>), nb, BS, 0, A);      \
     else TDGL_LAUNCH(ctx, K_BAND, by, (k_band_stage<false, false, LR>), nb, BS, 0, A);               \
   } while (0)
-  if (A.lr.mode == 1) TDGL_STAGE_LAUNCH(1);
+  if (A.lr.mode == 2) TDGL_STAGE_LAUNCH(2);
+  else if (A.lr.mode == 1) TDGL_STAGE_LAUNCH(1);
   else TDGL_STAGE_LAUNCH(0);
 #undef TDGL_STAGE_LAUNCH
 }
@@ -520,7 +526,6 @@ void band_euler(Ctx *ctx, int mu) {
   }
   launch_stage(ctx, A);
   if (ctx->P.rotframe && noise) {   // the low-passed rate, its rotation, then the turn back (bands.jl:336-339)
-    omega_faces(ctx);
     frame_smooth_rot(ctx, ctx->F[mu], ctx->P.dt);
     frame_rot(ctx, ctx->F[mu], -ctx->P.dt);
   }
@@ -540,6 +545,7 @@ void band_substeps(Ctx *ctx, int mu, int n) {
     StageArgs A = stage_base(ctx, mu, ctx->P.bcs[mu], (double)n);
     A.C = dst;
     A.S = src;
+    A.gfly = m > 1;
     A.Lx = L[0]; A.Ly = L[1]; A.Lz = L[2];
     A.h = h;
     if (rot) {
@@ -553,15 +559,10 @@ void band_substeps(Ctx *ctx, int mu, int n) {
       if (m == n) A.turn = 1;
     }
     launch_stage(ctx, A);
-    if (rot && noise && m == 1) {
-      omega_faces(ctx);
-      frame_smooth_rot(ctx, dst, h);
-    }
+    if (rot && noise && m == 1) frame_smooth_rot(ctx, dst, h);
     if (m < n) {
-      if (rot && m == 1) omega_faces(ctx);
       if (ex) link_op(ctx, LOP_ADVANCE, 0.0);
       if (rot) link_op(ctx, LOP_FRAME_LINKS, h);
-      ghosts(ctx, dst, L[0], L[1], L[2]);
     }
     src = dst;
   }
@@ -574,11 +575,14 @@ void band_rkl(Ctx *ctx, int mu, int ns) {
   const double q = kc ? P.rkc_q[mu] : (double)(ns * (ns + 1) / 2);
   const double h = P.dt / q;
   const cd *L[3] = {ctx->V[0], ctx->V[1], ctx->V[2]};
-  cd *buf[3] = {ctx->W, ctx->W2, ctx->F[mu]};
+  // the stages' destinations in turn, so that the last one is F[µ] (no copy at the end)
+  const int off = (2 - (ns - 1) % 3 + 3) % 3;
+  cd *ring[3] = {ctx->W, ctx->W2, ctx->F[mu]};
+  auto dest = [&](int j) { return ring[(j - 1 + off) % 3]; };
   const cd *A_ = ctx->G[mu], *B = ctx->G[mu];
-  cd *Cc = ctx->W;
+  cd *Cc = dest(1);
   // the links of stage j > 1 are the step's links rotated to the fraction c_{j−1} of the step, formed where the stage
-  // and its ghosts read them (no stored copy)
+  // reads them (no stored copy)
   LinkRot lr;
   memset(&lr, 0, sizeof(lr));
   for (int ax = 0; ax < 3; ax++) {
@@ -587,16 +591,16 @@ void band_rkl(Ctx *ctx, int mu, int ns) {
     lr.R[ax] = ctx->Rr[ax];
   }
   for (int j = 1; j <= ns; j++) {
-    Cc = buf[(j - 1) % 3];
+    Cc = dest(j);
     const cd *src = B;
     if (j == 1 && skq) {   // SK-ROCK for the phase: K₁ = E(Ψⁿ e^{iν₁δθ}) e^{i(κ₁−ν₁)δθ} (bands.jl:482-488)
-      sk_turn(ctx, ctx->W2, B, mu, P.rkc_sk[mu][0]);
-      ghosts(ctx, ctx->W2, L[0], L[1], L[2]);
-      src = ctx->W2;
+      sk_turn(ctx, dest(2), B, mu, P.rkc_sk[mu][0]);   // the second stage's destination is free until then
+      src = dest(2);
     }
     StageArgs A = stage_base(ctx, mu, P.bcs[mu], q);
     A.C = Cc;
     A.S = src;
+    A.gfly = j > 1 || skq;
     A.Lx = L[0]; A.Ly = L[1]; A.Lz = L[2];
     A.lr = lr;
     A.h = h;
@@ -619,64 +623,42 @@ void band_rkl(Ctx *ctx, int mu, int ns) {
     const bool late_turn = j == ns && rot && j == 1 && noise;   // the turn follows the low-passed rate
     if (j == ns && rot && !late_turn) A.turn = 1;
     launch_stage(ctx, A);
-    if (j == 1 && rot && noise) {
-      omega_faces(ctx);
-      frame_smooth_rot(ctx, Cc, h);
-    }
+    if (j == 1 && rot && noise) frame_smooth_rot(ctx, Cc, h);
     if (j == 1 && skq) sk_turn(ctx, Cc, Cc, mu, P.rkc_sk[mu][1] - P.rkc_sk[mu][0]);
     if (late_turn) frame_rot(ctx, Cc, -P.dt);
-    if (rot && j == 1 && ex && ns > 1) {
-      omega_faces(ctx);
-      link_op(ctx, LOP_LINK_RATE, P.dt);
-    }
-    if (j < ns) {
-      if (ex) {
-        const double c = kc ? P.rkc_c[mu][j - 1] : (double)(j * (j + 1)) / (double)(ns * (ns + 1));
-        if (rot) {
-          lr.mode = 1;
-          lr.c = c;
-        } else {
-          link_op(ctx, LOP_ROTFRAC, c);
-          for (int ax = 0; ax < 3; ax++) L[ax] = ctx->L[ax];
-        }
-      }
-      ghosts(ctx, Cc, L[0], L[1], L[2], &lr);
+    if (rot && j == 1 && ex && ns > 1) link_op(ctx, LOP_LINK_RATE, P.dt);
+    if (j < ns && ex) {
+      lr.mode = rot ? 1 : 2;
+      lr.c = kc ? P.rkc_c[mu][j - 1] : (double)(j * (j + 1)) / (double)(ns * (ns + 1));
     }
     A_ = B;
     B = Cc;
-  }
-  if (Cc != ctx->F[mu]) {
-    long long n = ctx->g.d.n();
-    TDGL_LAUNCH(ctx, K_COPY, 32.0 * n, k_copy_c, nblk(n, BS), BS, 0, ctx->F[mu], Cc, n);
   }
 }
 
 }  // namespace
 
-// Ω on the six faces copies the node inside (bands.jl:224-232, precedence x, y, z)
-void omega_faces(Ctx *ctx) {
-  const Geo &g = ctx->g;
-  Rng r0 = mkrng(0, 0, g.y1 + 1, g.y2, g.z1 + 1, g.z2);
-  Rng r1 = mkrng(g.x1, g.x2 + 1, 0, 0, g.z1 + 1, g.z2);
-  Rng r2 = mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, 0, 0);
-  r0.ni = 1; r1.nj = 1; r2.nk = 1;
-  TDGL_LAUNCH(ctx, K_OMEGA, 32.0 * r0.n(), k_omega_face, nblk(r0.n(), BS), BS, 0, ctx->Om, g.d, r0, 0, g.x1, g.x2);
-  TDGL_LAUNCH(ctx, K_OMEGA, 32.0 * r1.n(), k_omega_face, nblk(r1.n(), BS), BS, 0, ctx->Om, g.d, r1, 1, g.y1, g.y2);
-  TDGL_LAUNCH(ctx, K_OMEGA, 32.0 * r2.n(), k_omega_face, nblk(r2.n(), BS), BS, 0, ctx->Om, g.d, r2, 2, g.z1, g.z2);
+// The reference copies the last of an RKL/RKC band's buffers into F[µ] whole unless the stage count put it there: on
+// the nodes outside the block, which no stage writes, F is then the buffer's zeros.  The stages here end in F[µ]
+// themselves, so those nodes are cleared once, when a state came in from outside.
+void clear_outside(Ctx *ctx) {
+  const long long n = ctx->g.d.n();
+  for (int mu = 0; mu < ctx->N; mu++)
+    if (ctx->P.stages[mu] > 0 && (ctx->P.stages[mu] - 1) % 3 != 2) {
+      k_zero_outside<<<nblk(n, BS), BS, 0, ctx->stream>>>(ctx->F[mu], ctx->g);
+      ctx->launches++;
+    }
 }
 
-void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz, const LinkRot *lrp) {
+void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz) {
   const Geo &g = ctx->g;
-  LinkRot lr;
-  memset(&lr, 0, sizeof(lr));
-  if (lrp) lr = *lrp;
   if (g.x2 < g.x1 + 1 || g.y2 < g.y1 + 1 || g.z2 < g.z1 + 1) {   // a block one cell thick: the passes read ghosts
     Rng r0 = mkrng(1, 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
     Rng r1 = mkrng(g.x1, g.x2 + 1, 1, 1, g.z1, g.z2 + 1);
     Rng r2 = mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, 1, 1);
-    TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r0.n(), k_ghost_face, nblk(r0.n(), BS), BS, 0, X, Lx, g.d, r0, 0, g.x1, g.x2, lr);
-    TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r1.n(), k_ghost_face, nblk(r1.n(), BS), BS, 0, X, Ly, g.d, r1, 1, g.y1, g.y2, lr);
-    TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r2.n(), k_ghost_face, nblk(r2.n(), BS), BS, 0, X, Lz, g.d, r2, 2, g.z1, g.z2, lr);
+    TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r0.n(), k_ghost_face, nblk(r0.n(), BS), BS, 0, X, Lx, g.d, r0, 0, g.x1, g.x2);
+    TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r1.n(), k_ghost_face, nblk(r1.n(), BS), BS, 0, X, Ly, g.d, r1, 1, g.y1, g.y2);
+    TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r2.n(), k_ghost_face, nblk(r2.n(), BS), BS, 0, X, Lz, g.d, r2, 2, g.z1, g.z2);
     return;
   }
   ShellArgs A;
@@ -688,7 +670,6 @@ void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz, const Lin
   A.ny_face = 2 * ni * (nk - 2);
   A.n = A.nz_face + A.ny_face + 2 * (nj - 2) * (nk - 2);
   A.d = g.d;
-  A.lr = lr;
   // per shell point: the point, its link and the inside value(s) it reads (up to three of each on edges)
   TDGL_LAUNCH(ctx, K_GHOST, 48.0 * A.n, k_ghost_shell, nblk(A.n, BS), BS, 0, A);
 }

@@ -84,6 +84,12 @@ struct Geo {
   Dim d;
 };
 
+// The frame rate Ω is stored on the interior nodes r only; a node on the block's faces has the value of the nearest
+// interior node (bands.jl:224-232 copies the faces x, then y, then z, which clamps each index).
+__device__ __forceinline__ long long om_at(const Dim &d, const Rng &r, int i, int j, int k) {
+  return d.at(min(max(i, r.i0), r.i0 + r.ni - 1), min(max(j, r.j0), r.j0 + r.nj - 1), min(max(k, r.k0), r.k0 + r.nk - 1));
+}
+
 struct BandPtrs {
   const cd *p[TDGL_MAXB];
 };
@@ -221,6 +227,7 @@ struct Ctx {
   double *th[3] = {}, *ph[3] = {}, *J[3] = {}, *h[3] = {};
   cd *U[3] = {}, *V[3] = {};
   bool have_state = false;
+  bool outside_state = false;   // the state came in since the last step (clear_outside is due)
   // workspaces of the band stages
   cd *W = nullptr, *W2 = nullptr, *L[3] = {}, *Rl[3] = {};
   double *Th = nullptr;   // the heat model's temperature field (node-shaped; terms.jl)
@@ -354,9 +361,8 @@ void field_kick(Ctx *ctx);
 
 // bands.cu
 int update_bands(Ctx *ctx);
-void omega_faces(Ctx *ctx);
-struct LinkRot;   // bands.cu: links read as given or rotated on the fly
-void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz, const LinkRot *lr = nullptr);
+void clear_outside(Ctx *ctx);   // F = 0 outside the block, once for a state that came in from outside
+void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz);
 void vacuum_zero(Ctx *ctx);   // neumann! on a sculpted sample: F = 0 on every vacuum node, ghosts included
 // field.cu
 void supercurrent_increment(Ctx *ctx);

@@ -172,18 +172,23 @@ __device__ __forceinline__ void field_kick_b(const Blk bk, FKArgs const &K, Nois
   K.ph[ax][o] += amp * n;
 }
 
-// the smoothing sweep of the frame rate (bands.jl:255-261): Ω ← Ω/2 + (Σ six neighbours of the copy T)/12
-__device__ __forceinline__ void omega_smooth_b(const Blk bk, double * const &Om, const double * const &T, Rng const &r, Dim const &d);
-__global__ void k_omega_smooth(double *Om, const double *T, Rng r, Dim d) { omega_smooth_b(TDGL_BLK, Om, T, r, d); }
+// a smoothing sweep of the frame rate (bands.jl:255-261): Om ← T/2 + (Σ six neighbours of T)/12, T and Om two
+// buffers in turn (no copy), the faces read as the node inside (no face passes); the second sweep also turns the band,
+// C ← C e^{−iω̂h} (C null: none).  Six launches and two copies became two launches.
+__device__ __forceinline__ void omega_smooth_b(const Blk bk, double * const &Om, const double * const &T, cd * const &Cc, double const &h, Rng const &r, Dim const &d);
+__global__ void k_omega_smooth(double *Om, const double *T, cd *Cc, double h, Rng r, Dim d) { omega_smooth_b(TDGL_BLK, Om, T, Cc, h, r, d); }
 TDGL_MERGEABLE(k_omega_smooth, omega_smooth_b, 256, 1, false);
-__device__ __forceinline__ void omega_smooth_b(const Blk bk, double * const &Om, const double * const &T, Rng const &r, Dim const &d) {
+__device__ __forceinline__ void omega_smooth_b(const Blk bk, double * const &Om, const double * const &T, cd * const &Cc, double const &h, Rng const &r, Dim const &d) {
   const long long t = (long long)bk.x * blockDim.x + threadIdx.x;
   if (t >= r.n()) return;
   int i, j, k;
   rng_ijk(r, t, i, j, k);
-  const long long o = d.at(i, j, k), sy = d.n1, sz = (long long)d.n1 * d.n2;
-  const double nb = ((T[o + 1] + T[o - 1]) + (T[o + sy] + T[o - sy])) + (T[o + sz] + T[o - sz]);
-  Om[o] = 0.5 * T[o] + nb / 12;
+  const long long o = d.at(i, j, k);
+  auto at = [&](int a, int b, int c) { return T[om_at(d, r, a, b, c)]; };
+  const double nb = ((at(i + 1, j, k) + at(i - 1, j, k)) + (at(i, j + 1, k) + at(i, j - 1, k))) + (at(i, j, k + 1) + at(i, j, k - 1));
+  const double w = 0.5 * T[o] + nb / 12;
+  Om[o] = w;
+  if (Cc) Cc[o] = cmul(Cc[o], ccis(-(w * h)));
 }
 
 // C ← C e^{−iω̂h} on the interior (the frame term as a rotation, bands.jl:262-270)
@@ -229,16 +234,11 @@ void sk_turn(Ctx *ctx, cd *D, const cd *X, int mu, double c) {
               ctx->P.bcs[mu].gamma2, ctx->P.noise_gamma[mu], c, r, ctx->g.d);
 }
 
-// the low-passed frame rate (Ω of the stage already stored, the faces copied): two sweeps, then C ← C e^{−iω̂h}
+// the low-passed frame rate (Ω of the stage already stored): two sweeps, the second with C ← C e^{−iω̂h}
 void frame_smooth_rot(Ctx *ctx, cd *Cc, double h) {
   const Rng r = interior(ctx->g);
-  const long long n = ctx->g.d.n();
-  for (int pass = 0; pass < 2; pass++) {
-    cudaMemcpyAsync(ctx->Oms, ctx->Om, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream);   // errors surface at the sync
-    TDGL_LAUNCH(ctx, K_OMEGA, 64.0 * r.n(), k_omega_smooth, nblk(r.n(), BS), BS, 0, ctx->Om, ctx->Oms, r, ctx->g.d);
-    omega_faces(ctx);
-  }
-  TDGL_LAUNCH(ctx, K_OMEGA, 40.0 * r.n(), k_frame_rot, nblk(r.n(), BS), BS, 0, Cc, ctx->Om, h, r, ctx->g.d);
+  TDGL_LAUNCH(ctx, K_OMEGA, 16.0 * r.n(), k_omega_smooth, nblk(r.n(), BS), BS, 0, ctx->Oms, ctx->Om, nullptr, 0.0, r, ctx->g.d);
+  TDGL_LAUNCH(ctx, K_OMEGA, 48.0 * r.n(), k_omega_smooth, nblk(r.n(), BS), BS, 0, ctx->Om, ctx->Oms, Cc, h, r, ctx->g.d);
 }
 
 void frame_rot(Ctx *ctx, cd *Cc, double h) {
