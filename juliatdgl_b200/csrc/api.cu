@@ -268,11 +268,7 @@ static int step_body(Ctx *ctx) {
     default: break;
   }
   if (rc) return rc;
-  links_curl(ctx);
-  field_bc(ctx);
-  for (int mu = 0; mu < ctx->N; mu++) ghosts(ctx, ctx->F[mu], ctx->U[0], ctx->U[1], ctx->U[2]);
-  if (ctx->vac) vacuum_zero(ctx);   // neumann! (field.jl:235-244)
-  advance_copy(ctx);
+  finish_step(ctx);
   ctx->steps++;
   return 0;
 }

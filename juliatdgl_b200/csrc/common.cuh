@@ -363,13 +363,11 @@ void field_kick(Ctx *ctx);
 int update_bands(Ctx *ctx);
 void clear_outside(Ctx *ctx);   // F = 0 outside the block, once for a state that came in from outside
 void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz);
-void vacuum_zero(Ctx *ctx);   // neumann! on a sculpted sample: F = 0 on every vacuum node, ghosts included
+void vacuum_zero(Ctx *ctx);   // neumann! on a sculpted sample: F = 0 on every vacuum node
 // field.cu
 void supercurrent_increment(Ctx *ctx);
 void scale_increment(Ctx *ctx);
-void links_curl(Ctx *ctx);
-void field_bc(Ctx *ctx);   // H, HJ and the ramp fraction from ctx->ss_cur
-void advance_copy(Ctx *ctx);
+void finish_step(Ctx *ctx);   // links!, curl_h!, field_bc!, neumann!, advance!
 void advance_swap(Ctx *ctx);          // the host half of advance!: θ↔φ and V↔U by pointer
 // sep.cu
 int sep_create(Ctx *ctx);

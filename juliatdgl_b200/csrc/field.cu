@@ -3,11 +3,9 @@
 //   k_current_increment  supercurrent! (:19-46) fused with field_increment! (:84-102): J on each link is computed,
 //                        stored (the State carries it) and used at once for φ = θ + d1 τ J − s·Δh
 //   k_scale              scale_increment! (gtdgl/src/implicit.jl:337-342)
-//   k_links_curl         links! (:105-121) and curl_h! (:124-137) in one launch over their six ranges
-//   k_face_h             field_bc! (:189-228) with _open_add! (gtdgl/src/openbc.jl:210-223): each face point
-//                        evaluates the reference's sequence of face writes itself, so the precedence of the
-//                        overlapping `.=` statements is kept without ordering the threads
-//   k_advance            advance! (:248-263): G ← F on the block (θ/φ and V/U swap by pointer)
+//   k_finish             the end of the step in one launch: links! (:105-121), curl_h! (:124-137), field_bc!
+//                        (:189-228) with _open_add! (gtdgl/src/openbc.jl:210-223), neumann! (:231-246) and advance!
+//                        (:248-263; θ/φ and V/U swap by pointer)
 #include "common.cuh"
 #include "merge.cuh"
 
@@ -113,54 +111,38 @@ __device__ __forceinline__ void scale_b(const Blk bk, ScaleArgs const &A) {
   A.ph[ax][o] = A.th[ax][o] + (A.ph[ax][o] - A.th[ax][o]) / A.D[ax][o];
 }
 
-struct LCArgs {
+// The end of the step, one item per thread over sixteen ranges (the items of one range are whole warps but for its
+// ends): links U = e^{−iφ} (0..2), the curl on the inner plaquettes (3..5), the outer faces of h (6..14: per
+// component the k faces, the j faces and the i faces), the block's nodes of every band (15).  No item reads what
+// another writes: the faces of h are disjoint from the plaquettes of the curl, the ghosts take their links from φ
+// (the same e^{−iφ}) and read nodes inside the block, which no item writes in F.
+// What bounds it: an FP64 sincos per link on large grids; on small ones it is one launch where the links with the
+// curl, the faces of h, the ghosts of each band and the copy of advance! were N + 3, each waiting for the one before.
+// 40 steps took 2709 µs instead of 2811 (12×8×4 cells), 3597 instead of 3782 (64×32×8), 7638 instead of 7893
+// (192×64×16), 245.9 ms instead of 250.0 (the 256×128×32 ramp).  The ghosts are a call, not inlined, and the registers
+// are held to 32: inlined (110 registers) the links lost their occupancy and the 192×64×16 cycle took 8252 µs.
+struct FinArgs {
   const double *ph[3];
   cd *U[3];
   double *h[3];
-  Rng r[6];
-  long long off[7];
-  Dim d;
   double dx, dy, dz;
-};
-
-__device__ __forceinline__ void links_curl_b(const Blk bk, LCArgs const &A);
-__global__ void k_links_curl(LCArgs A) { links_curl_b(TDGL_BLK, A); }
-TDGL_MERGEABLE(k_links_curl, links_curl_b, BS, 1, false);
-__device__ __forceinline__ void links_curl_b(const Blk bk, LCArgs const &A) {
-  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
-  if (t >= A.off[6]) return;
-  int q = 0;
-  while (t >= A.off[q + 1]) q++;
-  t -= A.off[q];
-  int i, j, k;
-  rng_ijk(A.r[q], t, i, j, k);
-  const Dim d = A.d;
-  const long long o = d.at(i, j, k);
-  const long long sx = 1, sy = d.n1, sz = (long long)d.n1 * d.n2;
-  const double *px = A.ph[0], *py = A.ph[1], *pz = A.ph[2];
-  if (q < 3) {
-    A.U[q][o] = ccis(-A.ph[q][o]);
-  } else if (q == 3) {
-    A.h[0][o] = ((pz[o + sy] - pz[o]) - py[o + sz] + py[o]) / (A.dy * A.dz);
-  } else if (q == 4) {
-    A.h[1][o] = ((px[o + sz] - px[o]) - pz[o + sx] + pz[o]) / (A.dz * A.dx);
-  } else {
-    A.h[2][o] = ((py[o + sx] - py[o]) - px[o + sy] + px[o]) / (A.dx * A.dy);
-  }
-}
-
-struct FaceArgs {
-  double *h[3];
+  Rng r[16];
+  long long off[17];
+  Dim d;
+  // field_bc!
   const double *bar[6];     // hy_z, hy_y, hz_z, hz_y, hz_x, hy_x
   const double *oo[3], *on[3];
   const StepScal *cur;      // H, HJ and the ramp fraction of this step
   int bc, open;
   int Nx, Ny, Nz;
-  Rng r[9];                 // per component: k faces, j faces (k inner), i faces (j, k inner)
-  long long off[10];
-  Dim d;
+  // neumann! and advance!
+  cd *G[TDGL_MAXB], *F[TDGL_MAXB];
+  int N;
+  int x1, x2, y1, y2, z1, z2;
+  const uint8_t *vac;       // a sculpted sample: F = 0 on every vacuum node (range 15 is then the whole grid)
 };
 
+// advance! alone, for blocks one cell thick
 struct AdvArgs {
   cd *G[TDGL_MAXB];
   const cd *F[TDGL_MAXB];
@@ -236,70 +218,18 @@ void scale_increment(Ctx *ctx) {
   TDGL_LAUNCH(ctx, K_SCALE, 32.0 * n, k_scale, nblk(n, BS), BS, 0, A);
 }
 
-void links_curl(Ctx *ctx) {
-  const Geo &g = ctx->g;
-  LCArgs A;
+void advance_swap(Ctx *ctx) {
   for (int ax = 0; ax < 3; ax++) {
-    A.ph[ax] = ctx->ph[ax]; A.U[ax] = ctx->U[ax]; A.h[ax] = ctx->h[ax];
+    std::swap(ctx->th[ax], ctx->ph[ax]);
+    std::swap(ctx->V[ax], ctx->U[ax]);
   }
-  A.r[0] = mkrng(1, g.Nx, 2, g.Ny, 2, g.Nz);
-  A.r[1] = mkrng(2, g.Nx, 1, g.Ny, 2, g.Nz);
-  A.r[2] = mkrng(2, g.Nx, 2, g.Ny, 1, g.Nz);
-  A.r[3] = mkrng(2, g.Nx, 2, g.Ny - 1, 2, g.Nz - 1);
-  A.r[4] = mkrng(2, g.Nx - 1, 2, g.Ny, 2, g.Nz - 1);
-  A.r[5] = mkrng(2, g.Nx - 1, 2, g.Ny - 1, 2, g.Nz);
-  A.off[0] = 0;
-  for (int q = 0; q < 6; q++) A.off[q + 1] = A.off[q] + A.r[q].n();
-  A.d = g.d;
-  A.dx = g.dx; A.dy = g.dy; A.dz = g.dz;
-  const double nl = (double)A.off[3], nh = (double)(A.off[6] - A.off[3]);
-  TDGL_LAUNCH(ctx, K_LINKSCURL, 24.0 * nl + 8.0 * nh, k_links_curl, nblk(A.off[6], BS), BS, 0, A);
+  ctx->parity ^= 1;
 }
 
-// Face points: every point of the shell of each h array, each exactly once; each evaluates the final value of
-// field_bc! (field.jl:189-228) and _open_add! (openbc.jl:210-223) at that point.
-__global__ void k_face_h_shell(FaceArgs A);
-
-void field_bc(Ctx *ctx) {
-  const Geo &g = ctx->g;
-  FaceArgs A;
-  for (int c = 0; c < 3; c++) {
-    A.h[c] = ctx->h[c];
-    A.oo[c] = nullptr;
-    A.on[c] = nullptr;
-  }
-  for (int q = 0; q < 6; q++) A.bar[q] = ctx->bar[q];
-  A.cur = ctx->ss_cur;
-  A.bc = ctx->P.selffield_bc;
-  A.open = A.bc == TDGL_BC_OPEN;
-  A.Nx = g.Nx; A.Ny = g.Ny; A.Nz = g.Nz;
-  int shp[3][3] = {{g.Nx + 1, g.Ny, g.Nz}, {g.Nx, g.Ny + 1, g.Nz}, {g.Nx, g.Ny, g.Nz + 1}};
-  for (int c = 0; c < 3; c++) shell(shp[c][0], shp[c][1], shp[c][2], &A.r[3 * c]);
-  A.off[0] = 0;
-  for (int q = 0; q < 9; q++) A.off[q + 1] = A.off[q] + A.r[q].n();
-  A.d = g.d;
-  if (A.open) open_face_args(ctx, A.oo, A.on);
-  // the shells are described with far faces at local index 2; k_face_h_shell maps them
-  TDGL_LAUNCH(ctx, K_FACEH, (A.open ? 32.0 : 16.0) * A.off[9], k_face_h_shell, nblk(A.off[9], BS), BS, 0, A);
-}
-
-__device__ __forceinline__ void face_h_shell_b(const Blk bk, FaceArgs const &A);
-__global__ void k_face_h_shell(FaceArgs A) { face_h_shell_b(TDGL_BLK, A); }
-TDGL_MERGEABLE(k_face_h_shell, face_h_shell_b, BS, 1, false);
-__device__ __forceinline__ void face_h_shell_b(const Blk bk, FaceArgs const &A) {
-  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
-  if (t >= A.off[9]) return;
-  int q = 0;
-  while (t >= A.off[q + 1]) q++;
-  long long tt = t - A.off[q];
-  int i, j, k;
-  rng_ijk(A.r[q], tt, i, j, k);
-  const int comp = q / 3, part = q % 3;
+// one face point of h: the sequence of field_bc!'s face writes (field.jl:189-228) and _open_add! (openbc.jl:210-223)
+// as it ends at this point, so that the precedence of the overlapping `.=` statements needs no order of the threads
+__device__ __forceinline__ void face_point(const FinArgs &A, int comp, int i, int j, int k) {
   const int Nx = A.Nx, Ny = A.Ny, Nz = A.Nz;
-  const int ext[3][3] = {{Nx + 1, Ny, Nz}, {Nx, Ny + 1, Nz}, {Nx, Ny, Nz + 1}};
-  if (part == 0) k = face_of(k, ext[comp][2]);
-  else if (part == 1) j = face_of(j, ext[comp][1]);
-  else i = face_of(i, ext[comp][0]);
   const long long o = A.d.at(i, j, k);
   const double H = A.cur->H, HJ = A.cur->HJ, fr = A.cur->open_fr;
   double v = A.h[comp][o];
@@ -340,25 +270,130 @@ __device__ __forceinline__ void face_h_shell_b(const Blk bk, FaceArgs const &A) 
   A.h[comp][o] = v;
 }
 
-void advance_swap(Ctx *ctx) {
-  for (int ax = 0; ax < 3; ax++) {
-    std::swap(ctx->th[ax], ctx->ph[ax]);
-    std::swap(ctx->V[ax], ctx->U[ax]);
-  }
-  ctx->parity ^= 1;
+// The three face passes of ghosts! (bands.jl:524-539) at a point of the block's shell: the writes that reach it in the
+// reference's order (x faces, then y, then z).  A z-face point takes the z pass over the value the y or x pass left at
+// z1+1 / z2, a y-face point (k inside) the y pass over the x pass's value, an x-face point (j, k inside) the x pass.
+__device__ __noinline__ cd ghost_point(const FinArgs &A, const cd *X, int i, int j, int k) {
+  const Dim d = A.d;
+  const int x1 = A.x1, x2 = A.x2, y1 = A.y1, y2 = A.y2, z1 = A.z1, z2 = A.z2;
+  auto lk = [&](int ax, long long q) { return ccis(-A.ph[ax][q]); };
+  auto after_x = [&](int i, int j, int k) -> cd {
+    if (i == x1) return cmul(lk(0, d.at(x1, j, k)), X[d.at(x1 + 1, j, k)]);
+    if (i == x2 + 1) return cmul(cconj(lk(0, d.at(x2, j, k))), X[d.at(x2, j, k)]);
+    return X[d.at(i, j, k)];
+  };
+  auto after_y = [&](int i, int j, int k) -> cd {
+    if (j == y1) return cmul(lk(1, d.at(i, y1, k)), after_x(i, y1 + 1, k));
+    if (j == y2 + 1) return cmul(cconj(lk(1, d.at(i, y2, k))), after_x(i, y2, k));
+    return after_x(i, j, k);
+  };
+  if (k == z1) return cmul(lk(2, d.at(i, j, z1)), after_y(i, j, z1 + 1));
+  if (k == z2 + 1) return cmul(cconj(lk(2, d.at(i, j, z2))), after_y(i, j, z2));
+  return after_y(i, j, k);
 }
 
-void advance_copy(Ctx *ctx) {
+__device__ __forceinline__ void finish_b(const Blk bk, FinArgs const &A);
+__global__ void __launch_bounds__(BS, 8) k_finish(const __grid_constant__ FinArgs A) { finish_b(TDGL_BLK, A); }
+TDGL_MERGEABLE(k_finish, finish_b, BS, 6, false);
+__device__ __forceinline__ void finish_b(const Blk bk, FinArgs const &A) {
+  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
+  if (t >= A.off[16]) return;
+  int q = 0;
+  while (t >= A.off[q + 1]) q++;
+  t -= A.off[q];
+  int i, j, k;
+  rng_ijk(A.r[q], t, i, j, k);
+  const Dim d = A.d;
+  if (q >= 6 && q < 15) {   // the shells list the far faces at index 2
+    const int comp = (q - 6) / 3, part = (q - 6) % 3;
+    const int far = part == 0 ? (comp == 2 ? A.Nz + 1 : A.Nz) : part == 1 ? (comp == 1 ? A.Ny + 1 : A.Ny)
+                                                                          : (comp == 0 ? A.Nx + 1 : A.Nx);
+    if (part == 0) k = face_of(k, far);
+    else if (part == 1) j = face_of(j, far);
+    else i = face_of(i, far);
+    face_point(A, comp, i, j, k);
+    return;
+  }
+  const long long o = d.at(i, j, k);
+  const long long sx = 1, sy = d.n1, sz = (long long)d.n1 * d.n2;
+  const double *px = A.ph[0], *py = A.ph[1], *pz = A.ph[2];
+  if (q < 3) {
+    A.U[q][o] = ccis(-A.ph[q][o]);
+  } else if (q == 3) {
+    A.h[0][o] = ((pz[o + sy] - pz[o]) - py[o + sz] + py[o]) / (A.dy * A.dz);
+  } else if (q == 4) {
+    A.h[1][o] = ((px[o + sz] - px[o]) - pz[o + sx] + pz[o]) / (A.dz * A.dx);
+  } else if (q == 5) {
+    A.h[2][o] = ((py[o + sx] - py[o]) - px[o + sy] + px[o]) / (A.dx * A.dy);
+  } else {
+    const bool block = i >= A.x1 && i <= A.x2 + 1 && j >= A.y1 && j <= A.y2 + 1 && k >= A.z1 && k <= A.z2 + 1;
+    const bool shell = i == A.x1 || i == A.x2 + 1 || j == A.y1 || j == A.y2 + 1 || k == A.z1 || k == A.z2 + 1;
+    const bool vac = A.vac && A.vac[o];
+    for (int mu = 0; mu < A.N; mu++) {
+      if (!block) {   // with vacuum only
+        if (vac) A.F[mu][o] = mkc(0.0, 0.0);
+        continue;
+      }
+      const cd v = vac ? mkc(0.0, 0.0) : shell ? ghost_point(A, A.F[mu], i, j, k) : A.F[mu][o];
+      if (shell || vac) A.F[mu][o] = v;
+      A.G[mu][o] = v;
+    }
+  }
+}
+
+// links!, curl_h!, field_bc! (H, HJ and the ramp fraction from ctx->ss_cur), neumann! and advance!
+void finish_step(Ctx *ctx) {
   const Geo &g = ctx->g;
-  AdvArgs A;
+  FinArgs A;
+  memset(&A, 0, sizeof(A));
+  for (int ax = 0; ax < 3; ax++) {
+    A.ph[ax] = ctx->ph[ax]; A.U[ax] = ctx->U[ax]; A.h[ax] = ctx->h[ax];
+  }
+  A.dx = g.dx; A.dy = g.dy; A.dz = g.dz;
+  A.r[0] = mkrng(1, g.Nx, 2, g.Ny, 2, g.Nz);
+  A.r[1] = mkrng(2, g.Nx, 1, g.Ny, 2, g.Nz);
+  A.r[2] = mkrng(2, g.Nx, 2, g.Ny, 1, g.Nz);
+  A.r[3] = mkrng(2, g.Nx, 2, g.Ny - 1, 2, g.Nz - 1);
+  A.r[4] = mkrng(2, g.Nx - 1, 2, g.Ny, 2, g.Nz - 1);
+  A.r[5] = mkrng(2, g.Nx - 1, 2, g.Ny - 1, 2, g.Nz);
+  const int shp[3][3] = {{g.Nx + 1, g.Ny, g.Nz}, {g.Nx, g.Ny + 1, g.Nz}, {g.Nx, g.Ny, g.Nz + 1}};
+  for (int c = 0; c < 3; c++) shell(shp[c][0], shp[c][1], shp[c][2], &A.r[6 + 3 * c]);
+  for (int q = 0; q < 6; q++) A.bar[q] = ctx->bar[q];
+  A.cur = ctx->ss_cur;
+  A.bc = ctx->P.selffield_bc;
+  A.open = A.bc == TDGL_BC_OPEN;
+  if (A.open) open_face_args(ctx, A.oo, A.on);
+  A.Nx = g.Nx; A.Ny = g.Ny; A.Nz = g.Nz;
   for (int mu = 0; mu < ctx->N; mu++) {
     A.G[mu] = ctx->G[mu];
     A.F[mu] = ctx->F[mu];
   }
   A.N = ctx->N;
-  A.r = mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
+  A.x1 = g.x1; A.x2 = g.x2; A.y1 = g.y1; A.y2 = g.y2; A.z1 = g.z1; A.z2 = g.z2;
+  A.vac = ctx->vac;
+  // a block one cell thick has no node inside: its face passes read each other's ghosts and run one after the other
+  const bool thin = g.x2 < g.x1 + 1 || g.y2 < g.y1 + 1 || g.z2 < g.z1 + 1;
+  A.r[15] = ctx->vac ? mkrng(1, g.Nx + 1, 1, g.Ny + 1, 1, g.Nz + 1) : mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
+  if (thin) A.r[15].ni = 0;
+  A.off[0] = 0;
+  for (int q = 0; q < 16; q++) A.off[q + 1] = A.off[q] + A.r[q].n();
   A.d = g.d;
-  TDGL_LAUNCH(ctx, K_ADVANCE, 32.0 * ctx->N * A.r.n(), k_advance, nblk(A.r.n(), BS), BS, 0, A);
+  const double nl = (double)A.off[3], nh = (double)(A.off[6] - A.off[3]), nf = (double)(A.off[15] - A.off[6]);
+  const double bytes = 24.0 * nl + 8.0 * nh + (A.open ? 32.0 : 16.0) * nf + 32.0 * ctx->N * A.r[15].n();
+  TDGL_LAUNCH(ctx, K_LINKSCURL, bytes, k_finish, nblk(A.off[16], BS), BS, 0, A);
+  if (thin) {
+    for (int mu = 0; mu < ctx->N; mu++) ghosts(ctx, ctx->F[mu], ctx->U[0], ctx->U[1], ctx->U[2]);
+    if (ctx->vac) vacuum_zero(ctx);
+    AdvArgs V;
+    for (int mu = 0; mu < ctx->N; mu++) {
+      V.G[mu] = ctx->G[mu];
+      V.F[mu] = ctx->F[mu];
+    }
+    V.N = ctx->N;
+    V.r = mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
+    V.d = g.d;
+    TDGL_LAUNCH(ctx, K_ADVANCE, 32.0 * ctx->N * V.r.n(), k_advance, nblk(V.r.n(), BS), BS, 0, V);
+  }
   advance_swap(ctx);
 }
 
