@@ -81,6 +81,14 @@ struct PlaneArgs {
   int jc, ppb;               // k_plane: output rows per chunk, planes per pass at most
 };
 
+// The three components' transforms of one direction, component blk.z, in one launch: each is far from filling the GPU
+// on the grids of the sweep, and as launches in line they each waited for the one before (40 steps: 2709 → 2160 µs on
+// 12×8×4 cells, 3597 → 2669 on 64×32×8, 7638 → 6679 on 192×64×16; the same bits).  Components whose grids differ
+// (planes, chunks) share the larger grid; a block beyond its component's chunks returns.
+struct PlaneMulti {
+  PlaneArgs c[3];
+};
+
 const int PL_JC = 48, PL_THREADS = 192, PL_PPB = 8;
 
 __device__ __forceinline__ void ld4(float *v, const float *p) {
@@ -145,15 +153,16 @@ struct Tile {
 // TA: output rows jo per register tile (tiles TA × 4).  Large planes take 4 (fewer shared loads per multiply-add);
 // small ones 2, so that a pass has more tiles for the block's threads and fewer registers keep more blocks per SM.
 template <class TIn, class TOut, class T, int TA>
-__device__ __forceinline__ void plane_b(const Blk bk, PlaneArgs const &A);
+__device__ __forceinline__ void plane_b(const Blk bk, PlaneMulti const &M);
 template <class TIn, class TOut, class T, int TA>
-__global__ void __launch_bounds__(PL_THREADS, TA == 2 ? 4 : 1) k_plane(PlaneArgs A) {
-  plane_b<TIn, TOut, T, TA>(TDGL_BLK, A);
+__global__ void __launch_bounds__(PL_THREADS, TA == 2 ? 4 : 1) k_plane(const __grid_constant__ PlaneMulti M) {
+  plane_b<TIn, TOut, T, TA>(TDGL_BLK, M);
 }
 TDGL_MERGEABLE((k_plane<double, double, double, 2>), (plane_b<double, double, double, 2>), PL_THREADS, 4, true);
 TDGL_MERGEABLE((k_plane<double, double, double, 4>), (plane_b<double, double, double, 4>), PL_THREADS, 1, true);
 template <class TIn, class TOut, class T, int TA>
-__device__ __forceinline__ void plane_b(const Blk bk, PlaneArgs const &A) {
+__device__ __forceinline__ void plane_b(const Blk bk, PlaneMulti const &M) {
+  const PlaneArgs &A = M.c[bk.z];
   if (A.done && *A.done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   // planes per pass: up to A.ppb (what the shared memory holds), as many as the block's share of the planes allows
@@ -168,6 +177,7 @@ __device__ __forceinline__ void plane_b(const Blk bk, PlaneArgs const &A) {
   T *Ins = M2s + (size_t)nk * KO;          // PPB × [nj_in][KP]
   T *O1s = Ins + (size_t)PPB * nj * KP;    // PPB × [KP][JC]
   const int jo0 = bk.y * JC;
+  if (jo0 >= A.nj_out) return;
   const T *M1t = (const T *)A.M1t, *M2t = (const T *)A.M2t;
   const int tid = threadIdx.x;
   const int pin = nj * KP, po1 = KP * JC;   // per-plane strides of Ins and O1s
@@ -1281,41 +1291,53 @@ void half_gemm(Ctx *ctx, const HalfArgs &A, bool fwd, const double *in64, const 
 }
 
 template <class TIn, class TOut, class T>
-void plane(Ctx *ctx, PlaneArgs A) {
-  const double bytes = (double)A.nplanes * ((double)A.nj_in * A.nk_in * sizeof(TIn) + (double)A.nj_out * A.nk_out * sizeof(TOut));
-  const int ngy = (A.nj_out + PL_JC - 1) / PL_JC;
-  // planes whose one-block transform would hold more than GB_ONEBLOCK of shared memory (at most two blocks per SM)
-  // take the batched products when the context has their buffer
-  const size_t one = plane_smem<T>(A.nj_in, A.nk_in, A.nk_out);
-  if (one > GB_ONEBLOCK && one <= 227 * 1024 && ctx->sep && ctx->sep->gtmp) {
-    plane_gemm<TIn, TOut, T>(ctx, A, (T *)ctx->sep->gtmp, bytes);
+void plane(Ctx *ctx, PlaneMulti M) {
+  const int cat = sizeof(T) == 8 ? K_TX64 : K_TX32;
+  double bytes[3], all = 0;
+  size_t one = 0;   // the largest component's shared memory in the one-block transform, one plane at a time
+  int njm = 0;
+  for (int c = 0; c < 3; c++) {
+    const PlaneArgs &A = M.c[c];
+    bytes[c] = (double)A.nplanes * ((double)A.nj_in * A.nk_in * sizeof(TIn) + (double)A.nj_out * A.nk_out * sizeof(TOut));
+    all += bytes[c];
+    one = std::max(one, plane_smem<T>(A.nj_in, A.nk_in, A.nk_out));
+    njm = std::max(njm, A.nj_out);
+  }
+  // planes whose one-block transform would hold more than GB_ONEBLOCK of shared memory (at most two blocks per SM), or
+  // would not fit one block, take two batched products through a plane-sized buffer when the context has one
+  if (one > GB_ONEBLOCK && ctx->sep && ctx->sep->gtmp) {
+    for (int c = 0; c < 3; c++) plane_gemm<TIn, TOut, T>(ctx, M.c[c], (T *)ctx->sep->gtmp, bytes[c]);
   } else if (one <= 227 * 1024) {
     // the output rows split evenly over the chunks (no chunk mostly empty); room for as many planes per pass as keep
     // the threads busy (at most PL_PPB; at most 56 KB of shared memory, four blocks per SM), used when a block has
     // several planes (a merged launch gives each context fewer blocks); persistent: a block keeps its basis chunks
-    // in shared memory for all its planes (about four blocks per SM in all).  Small planes take 2-row tiles.
-    const bool small = A.nj_out <= 2 * PL_JC;
-    A.jc = small ? rup4((A.nj_out + ngy - 1) / ngy) : PL_JC;
-    const int ta = small ? 2 : 4;
-    const int tiles = (A.jc / ta) * (std::max(rup4(A.nk_in), rup4(A.nk_out)) / 4);
-    A.ppb = std::max(1, std::min(PL_PPB, PL_THREADS / std::max(1, tiles)));
-    while (A.ppb > 1 && plane_smem<T>(A.nj_in, A.nk_in, A.nk_out, A.jc, A.ppb) > 56 * 1024) A.ppb--;
-    const size_t smem = plane_smem<T>(A.nj_in, A.nk_in, A.nk_out, A.jc, A.ppb);
+    // in shared memory for all its planes (about four blocks per SM a component).  Small planes take 2-row tiles.
+    const bool small = njm <= 2 * PL_JC;
     const int nsm = g_sm_count > 0 ? g_sm_count : 148;
-    dim3 grid(std::max(1, std::min((int)A.nplanes, (4 * nsm + ngy - 1) / ngy)), ngy);
-    const int cat = sizeof(T) == 8 ? K_TX64 : K_TX32;
-    if (small) TDGL_LAUNCH(ctx, cat, bytes, (k_plane<TIn, TOut, T, 2>), grid, PL_THREADS, smem, A);
-    else TDGL_LAUNCH(ctx, cat, bytes, (k_plane<TIn, TOut, T, 4>), grid, PL_THREADS, smem, A);
-  } else if (ctx->sep && ctx->sep->gtmp) {
-    // a plane too large for one block: two batched products through a plane-sized buffer
-    plane_gemm<TIn, TOut, T>(ctx, A, (T *)ctx->sep->gtmp, bytes);
+    size_t smem = 0;
+    int ngy = 1, gx = 1;
+    for (int c = 0; c < 3; c++) {
+      PlaneArgs &A = M.c[c];
+      const int ny = (A.nj_out + PL_JC - 1) / PL_JC;
+      A.jc = small ? rup4((A.nj_out + ny - 1) / ny) : PL_JC;
+      const int ta = small ? 2 : 4;
+      const int tiles = (A.jc / ta) * (std::max(rup4(A.nk_in), rup4(A.nk_out)) / 4);
+      A.ppb = std::max(1, std::min(PL_PPB, PL_THREADS / std::max(1, tiles)));
+      while (A.ppb > 1 && plane_smem<T>(A.nj_in, A.nk_in, A.nk_out, A.jc, A.ppb) > 56 * 1024) A.ppb--;
+      smem = std::max(smem, plane_smem<T>(A.nj_in, A.nk_in, A.nk_out, A.jc, A.ppb));
+      ngy = std::max(ngy, ny);
+      gx = std::max(gx, std::min((int)A.nplanes, (4 * nsm + ny - 1) / ny));
+    }
+    const dim3 grid(gx, ngy, 3);
+    if (small) TDGL_LAUNCH(ctx, cat, all, (k_plane<TIn, TOut, T, 2>), grid, PL_THREADS, smem, M);
+    else TDGL_LAUNCH(ctx, cat, all, (k_plane<TIn, TOut, T, 4>), grid, PL_THREADS, smem, M);
   } else {
-    // a plane too large for one block, without the buffer: chunked sums (sep_create checked that these fit)
-    A.jc = PL_JC;
-    A.ppb = 1;
-    dim3 grid(A.nplanes, ngy);
-    TDGL_LAUNCH(ctx, sizeof(T) == 8 ? K_TX64 : K_TX32, bytes, (k_plane_tiled<TIn, TOut, T>), grid, PT_THREADS,
-                tiled_smem<T>(A.nk_out), A);
+    // planes too large for one block, without the buffer: chunked sums (sep_create checked that these fit)
+    for (int c = 0; c < 3; c++) {
+      PlaneArgs &A = M.c[c];
+      dim3 grid(A.nplanes, (A.nj_out + PL_JC - 1) / PL_JC);
+      TDGL_LAUNCH(ctx, cat, bytes[c], (k_plane_tiled<TIn, TOut, T>), grid, PT_THREADS, tiled_smem<T>(A.nk_out), A);
+    }
   }
 }
 
@@ -1351,9 +1373,10 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
   const int nx = S->nx, ny = S->ny, nz = S->nz;
   const long long n2 = g.Ny + 1, n3 = g.Nz + 1, ps = n2 * n3, P = S->P;
   // the ranges (implicit.jl:52) start at i = j = k = 2 (0-based plane 1, row 1, column 1)
-  auto fwd = [&](const double *in, int nj, int nk, const T *M1t, const T *M2t, int njo, int nko, int jo_off, int ko_off,
+  PlaneMulti F, I;
+  auto fwd = [&](int c, const double *in, int nj, int nk, const T *M1t, const T *M2t, int njo, int nko, int jo_off, int ko_off,
                  T *hat, int nplanes) {
-    PlaneArgs A;
+    PlaneArgs &A = F.c[c];
     A.in = in; A.in_base = ps; A.in_ps = ps; A.in_ld = (int)n2; A.in_j0 = 1; A.in_k0 = 1;
     A.nj_in = nj; A.nk_in = nk;
     A.M1t = M1t; A.M2t = M2t;
@@ -1361,11 +1384,10 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
     A.out = hat; A.out_base = 0; A.out_ps = P; A.out_ld = ny; A.out_j0 = jo_off; A.out_k0 = ko_off;
     A.nplanes = nplanes;
     A.done = done;
-    plane<double, T, T>(ctx, A);
   };
-  auto inv = [&](const T *hat, int nj, int nk, int j_off, int k_off, const T *M1t, const T *M2t, int njo, int nko, double *out,
-                 int nplanes) {
-    PlaneArgs A;
+  auto inv = [&](int c, const T *hat, int nj, int nk, int j_off, int k_off, const T *M1t, const T *M2t, int njo, int nko,
+                 double *out, int nplanes) {
+    PlaneArgs &A = I.c[c];
     A.in = hat; A.in_base = 0; A.in_ps = P; A.in_ld = ny; A.in_j0 = j_off; A.in_k0 = k_off;
     A.nj_in = nj; A.nk_in = nk;
     A.M1t = M1t; A.M2t = M2t;
@@ -1373,7 +1395,6 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
     A.out = out; A.out_base = ps; A.out_ps = ps; A.out_ld = (int)n2; A.out_j0 = 1; A.out_k0 = 1;
     A.nplanes = nplanes;
     A.done = done;
-    plane<T, double, T>(ctx, A);
   };
   if constexpr (sizeof(T) == 4) {
     if (r32) {   // the mirror-halved FP32 transforms: one launch per direction for the three components
@@ -1436,13 +1457,15 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
   }
   // forward: X by (Vy, Vz), Y by (Uy, Vz), Z by (Vy, Uz) (implicit.jl:63-65 without the x transform).  The
   // transforms take the transposed matrices: forward V → Vt, inverse V' → V.
-  fwd(r[0], ny, nz, b[1].Vt, b[2].Vt, ny, nz, 0, 0, w.Xh, nx - 1);
-  fwd(r[1], ny - 1, nz, b[1].Ut, b[2].Vt, ny - 1, nz, 1, 0, w.Yh, nx);
-  fwd(r[2], ny, nz - 1, b[1].Vt, b[2].Ut, ny, nz - 1, 0, 1, w.Zh, nx);
+  fwd(0, r[0], ny, nz, b[1].Vt, b[2].Vt, ny, nz, 0, 0, w.Xh, nx - 1);
+  fwd(1, r[1], ny - 1, nz, b[1].Ut, b[2].Vt, ny - 1, nz, 1, 0, w.Yh, nx);
+  fwd(2, r[2], ny, nz - 1, b[1].Vt, b[2].Ut, ny, nz - 1, 0, 1, w.Zh, nx);
+  plane<double, T, T>(ctx, F);
   linesolve<T>(ctx, S, w, done);
-  inv(w.Xh, ny, nz, 0, 0, b[1].V, b[2].V, ny, nz, z[0], nx - 1);
-  inv(w.Yh, ny - 1, nz, 1, 0, b[1].U, b[2].V, ny - 1, nz, z[1], nx);
-  inv(w.Zh, ny, nz - 1, 0, 1, b[1].V, b[2].U, ny, nz - 1, z[2], nx);
+  inv(0, w.Xh, ny, nz, 0, 0, b[1].V, b[2].V, ny, nz, z[0], nx - 1);
+  inv(1, w.Yh, ny - 1, nz, 1, 0, b[1].U, b[2].V, ny - 1, nz, z[1], nx);
+  inv(2, w.Zh, ny, nz - 1, 0, 1, b[1].V, b[2].U, ny, nz - 1, z[2], nx);
+  plane<T, double, T>(ctx, I);
 }
 
 // the mode-space arrays of one precision; the FP64 factorisation of the line solves is allocated with the FP64 work

@@ -1,0 +1,29 @@
+"""The separable inverse at the edges of its transforms' tiles: extents where the components' row chunks differ in number
+or kind (48 | 49 and 96 | 97 rows), remainders of the register tiles, and the smallest planes; FP64 and FP32, against
+the oracle's dense three-axis transforms at the tolerances of the parity test."""
+import numpy as np
+import pytest
+
+import juliatdgl_b200 as T
+from juliatdgl_b200 import gpu
+from juliatdgl_b200.scheme import sep_unknowns
+from oracle import pyoracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("nx,ny,nz", [(5, 48, 3), (3, 96, 6), (9, 47, 17), (2, 2, 2), (20, 13, 4), (33, 5, 9)])
+def test_separable_inverse_sizes(nx, ny, nz, f32):
+    gr = T.Grid.make(nx, ny, nz, dx=0.5, buf=1)
+    md = T.two_band(xi_ratio=4.0, κ=2.0)
+    st = T.Stepper.make(md, gr, T.box_masks(gr), σvac=0.01 if f32 else None, pcg_f32=f32, selffield_bc="slab")
+    o = pyoracle.OracleStepper(st)
+    gs = gpu.GPUStepper(st)
+    try:
+        b = np.random.default_rng(5).standard_normal(sep_unknowns(gr))
+        ref = o.sep_apply(b, f32=False)
+        out = gs.sep_apply(b, f32=f32)
+    finally:
+        gs.close()
+    assert np.max(np.abs(out - ref)) / np.max(np.abs(ref)) <= (2e-6 if f32 else 1e-13)
