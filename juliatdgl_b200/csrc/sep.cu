@@ -51,8 +51,7 @@ struct SepDev {
   float *r32[3] = {};        // FP32 copy of the preconditioner's input (PCG with the FP32 preconditioner)
   bool tc = false;           // the FP32 preconditioner's plane transforms run on the tensor cores (sep_tc.cu)
   void *gtmp = nullptr;      // planes too large for one block: the first product of every plane (k_bgemm)
-  float *hx = nullptr, *ho = nullptr;   // the mirror-halved FP32 transforms of large planes: X / O2 and O1 per plane
-  long long hx_ps = 0, ho_ps = 0;       // their plane strides
+  HalfWork hw;               // the mirror-halved FP32 transforms of large planes (sep_half.cu; x[0] null: not taken)
   Work<double> wd;
   Work<float> wf;
 };
@@ -368,27 +367,11 @@ __device__ __forceinline__ void plane_tiled_b(const Blk bk, PlaneArgs const &A) 
 // R = C = 8⌈h/8⌉, JP = R0 + R1, KP = 8⌈n2/8⌉, KS = 4·odd ≥ C0 + C1 (conflict-free float4 rows).  The half
 // blocks are stored in global memory already padded this way ([h][8⌈h/8⌉] each), so each block copies one
 // contiguous image per axis with 16-byte cp.async.
-const int HX_THREADS = 256, HX_HALF = HX_THREADS / 2, HX_HWARPS = HX_HALF / 32, P32_KPAD = 52;
+const int HX_THREADS = 256, HX_HALF = HX_THREADS / 2, HX_HWARPS = HX_HALF / 32;
 
-__host__ __device__ inline int p32_ks(int KO) { return 4 * ((KO / 4) | 1); }
 // column c of X sits at xsw(c) in its row: the 8-column groups of consecutive column tiles (32 bytes apart) would
 // put tiles kt and kt + 4 on the same banks; columns ≥ 32 shift by 4 floats (rows have P32_KPAD = 52 ≥ 48 + 4)
 __host__ __device__ inline int xsw(int c) { return c + ((c >> 5) << 2); }
-
-struct HalfGeo {
-  int hS1, hD1, hS2, hD2, R0, R1, C0, C1, JP, KP, KS, XR;
-  __host__ __device__ HalfGeo(int n1, int n2) {
-    hS1 = (n1 + 1) / 2; hD1 = n1 / 2; hS2 = (n2 + 1) / 2; hD2 = n2 / 2;
-    R0 = rup8(hS1); R1 = rup8(hD1); C0 = rup8(hS2); C1 = rup8(hD2);
-    JP = R0 + R1; KP = rup8(n2); KS = p32_ks(C0 + C1); XR = n1 > JP ? n1 : JP;
-  }
-  __host__ __device__ size_t wfloats() const {
-    return (size_t)hS1 * R0 + (size_t)hD1 * R1 + (size_t)hS2 * C0 + (size_t)hD2 * C1;
-  }
-  __host__ __device__ size_t slot(int n1, int n2) const {   // one plane's XO, O1 and Stg, rounded to 16 bytes
-    return ((size_t)XR * P32_KPAD + (size_t)KP * JP + (size_t)n1 * n2 + 3) & ~(size_t)3;
-  }
-};
 
 size_t half_smem(int n1, int n2) {
   const HalfGeo G(n1, n2);
@@ -1107,189 +1090,6 @@ void plane_gemm(Ctx *ctx, const PlaneArgs &A, T *tmp, double bytes) {
   TDGL_LAUNCH(ctx, cat, bytes / 2, (k_bgemm<T, T, TOut, T>), g2, GB_THREADS, 0, G2);
 }
 
-// The mirror-halved FP32 transforms (as k_half32) of planes too large for one block: a pass that pairs the points
-// (forward) or gathers the modes in class order (inverse) into X, the row product and the column product of each
-// class as batched products (k_bgemm) on the half blocks, and a pass that scatters the modes (forward) or unpairs the
-// points (inverse).  Per plane: X (n1 × n2, class order, column-major), O1 (JP × n2), O2 (JP × (C0 + C1), in X's
-// buffer); the products sum in k_half32's order, so the results are its.
-template <bool FWD>
-__global__ void k_half_in(HalfArgs A, float *X, long long xps, const double *in64, const int *done) {
-  if (done && *done) return;
-  const HalfGeo G(A.n1, A.n2);
-  const int n1 = A.n1, n2 = A.n2;
-  const long long per = FWD ? (long long)G.hS1 * G.hS2 : (long long)n1 * n2;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= per * A.nplanes) return;
-  const long long q = t / per;
-  const int e = (int)(t % per);
-  float *x = X + q * xps;
-  if (FWD) {   // the four points of a mirror quadrant (p, qc) → its four class entries SS, SD, DS, DD
-    const double *in = in64 + A.in_base + q * A.in_ps + A.in_j0 + (long long)A.in_ld * A.in_k0;
-    const int qc = e % G.hS2, p = e / G.hS2, pp = n1 - 1 - p, qq = n2 - 1 - qc;
-    const bool rp = pp != p, cp = qq != qc;
-    const float a = (float)in[p + (long long)A.in_ld * qc];
-    const float b = rp ? (float)in[pp + (long long)A.in_ld * qc] : 0.f;
-    const float c = cp ? (float)in[p + (long long)A.in_ld * qq] : 0.f;
-    const float d = rp && cp ? (float)in[pp + (long long)A.in_ld * qq] : 0.f;
-    const float s0 = a + c, s1 = b + d, d0 = a - c, d1 = b - d;
-    x[p + (long long)n1 * qc] = s0 + s1;
-    if (cp) x[p + (long long)n1 * (G.hS2 + qc)] = d0 + d1;
-    if (rp) {
-      x[G.hS1 + p + (long long)n1 * qc] = s0 - s1;
-      if (cp) x[G.hS1 + p + (long long)n1 * (G.hS2 + qc)] = d0 - d1;
-    }
-  } else {     // X(r, c) = the mode of class order (r, c): even modes first
-    const float *in = A.in + A.in_base + q * A.in_ps + A.in_j0 + (long long)A.in_ld * A.in_k0;
-    const int r = e % n1, c = e / n1;
-    const int m = r < G.hS1 ? 2 * r : 2 * (r - G.hS1) + 1, mk = c < G.hS2 ? 2 * c : 2 * (c - G.hS2) + 1;
-    x[r + (long long)n1 * c] = in[m + (long long)A.in_ld * mk];
-  }
-}
-
-template <bool FWD>
-__global__ void k_half_out(HalfArgs A, const float *O2, long long ops, const int *done) {
-  if (done && *done) return;
-  const HalfGeo G(A.n1, A.n2);
-  const int n1 = A.n1, n2 = A.n2, JP = G.JP;
-  const long long per = FWD ? (long long)n1 * n2 : (long long)G.hS1 * G.hS2;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= per * A.nplanes) return;
-  const long long q = t / per;
-  const int e = (int)(t % per);
-  const float *o2 = O2 + q * ops;
-  if (FWD) {   // modes in order: row j from its class (even j: E row j/2, odd: O row R0 + j/2), likewise columns
-    float *out = (float *)A.out + A.out_base + q * A.out_ps + A.out_j0 + (long long)A.out_ld * A.out_k0;
-    const int j = e % n1, k = e / n1;
-    const int r = (j & 1) ? G.R0 + (j >> 1) : (j >> 1), c = (k & 1) ? G.C0 + (k >> 1) : (k >> 1);
-    out[j + (long long)A.out_ld * k] = o2[r + (long long)JP * c];
-  } else {     // unpair one mirror quadrant (p, qc) into its four points
-    double *out = (double *)A.out + A.out_base + q * A.out_ps + A.out_j0 + (long long)A.out_ld * A.out_k0;
-    const int p = e % G.hS1, qc = e / G.hS1, pp = n1 - 1 - p, qq = n2 - 1 - qc;
-    const bool rp = pp != p, cp = qq != qc;
-    const float ee = o2[p + (long long)JP * qc];
-    const float eo = cp ? o2[p + (long long)JP * (G.C0 + qc)] : 0.f;
-    const float oe = rp ? o2[G.R0 + p + (long long)JP * qc] : 0.f;
-    const float oo = rp && cp ? o2[G.R0 + p + (long long)JP * (G.C0 + qc)] : 0.f;
-    const float s0 = ee + oe, s1 = eo + oo, d0 = ee - oe, d1 = eo - oo;
-    const long long oq = (long long)A.out_ld * qc, oqq = (long long)A.out_ld * qq;
-    out[oq + p] = (double)(s0 + s1);
-    if (rp) out[oq + pp] = (double)(d0 + d1);
-    if (cp) {
-      out[oqq + p] = (double)(s0 - s1);
-      if (rp) out[oqq + pp] = (double)(d0 - d1);
-    }
-  }
-}
-
-// The same batched product with the tile shape as template parameters: BM × BN outputs per block, TM × TN per thread
-// (TM or TN = 8: two runs of 4, half a tile apart, so that the 16-byte shared loads of a quarter warp are one
-// contiguous row; 6: one run).  The mirror-halved products take 48 × 96 tiles (rows ⌈n/2⌉ = 144, columns n2 = 95) and
-// 96 × 48 tiles (rows JP = 288, columns 48), which divide them with almost no empty outputs; 96 threads each.
-template <int BM, int BN, int TM, int TN, class T>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN)) k_bgemm_t(BGemm G) {
-  constexpr int NT = (BM / TM) * (BN / TN), LA = GB_K * BM / NT, LB = GB_K * BN / NT;
-  if (G.done && *G.done) return;
-  __shared__ __align__(16) T As[GB_K][BM + 4];
-  __shared__ __align__(16) T Bs[GB_K][BN + 4];
-  const int tid = threadIdx.x, m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const long long q = blockIdx.z;
-  const T *Ap = (const T *)G.A + G.a_off + q * G.a_q;
-  const T *Bp = (const T *)G.B + G.b_off + q * G.b_q;
-  static_assert(NT % BM == 0 && NT % BN == 0 && NT % GB_K == 0, "tile loads: whole rows per pass");
-  const bool am = G.a_m == 1, bk = G.b_k == 1;
-  // element u of this thread's loads: A (m, k) = (tid % BM, tid / BM + u NT/BM) when a_m = 1, else
-  // (tid / 16 + u NT/16, tid % 16); B likewise
-  const int a_m0 = am ? tid % BM : tid / GB_K, a_k0 = am ? tid / BM : tid % GB_K;
-  const int a_dm = am ? 0 : NT / GB_K, a_dk = am ? NT / BM : 0;
-  const int b_n0 = bk ? tid / GB_K : tid % BN, b_k0 = bk ? tid % GB_K : tid / BN;
-  const int b_dn = bk ? NT / GB_K : 0, b_dk = bk ? 0 : NT / BN;
-  const int tm = tid % (BM / TM), tn = tid / (BM / TM);
-  auto row = [&](int a) { return TM == 8 ? (a < 4 ? 4 * tm + a : BM / 2 + 4 * tm + a - 4) : TM * tm + a; };
-  auto col = [&](int b) { return TN == 8 ? (b < 4 ? 4 * tn + b : BN / 2 + 4 * tn + b - 4) : TN * tn + b; };
-  T acc[TM][TN];
-#pragma unroll
-  for (int a = 0; a < TM; a++)
-#pragma unroll
-    for (int b = 0; b < TN; b++) acc[a][b] = T(0);
-  for (int k0 = 0; k0 < G.K; k0 += GB_K) {
-    __syncthreads();
-#pragma unroll 4
-    for (int u = 0; u < LA; u++) {
-      const int m = a_m0 + a_dm * u, k = a_k0 + a_dk * u;
-      const int gm = m0 + m, gk = k0 + k;
-      As[k][m] = (gm < G.M && gk < G.K) ? Ap[G.a_m * gm + G.a_k * gk] : T(0);
-    }
-#pragma unroll 4
-    for (int u = 0; u < LB; u++) {
-      const int n = b_n0 + b_dn * u, k = b_k0 + b_dk * u;
-      const int gn = n0 + n, gk = k0 + k;
-      Bs[k][n] = (gn < G.N && gk < G.K) ? Bp[G.b_k * gk + G.b_n * gn] : T(0);
-    }
-    __syncthreads();
-    const int kn = min(GB_K, G.K - k0);
-    for (int k = 0; k < kn; k++) {
-      T av[TM], bv[TN];
-#pragma unroll
-      for (int a = 0; a < TM; a++) av[a] = As[k][row(a)];
-#pragma unroll
-      for (int b = 0; b < TN; b++) bv[b] = Bs[k][col(b)];
-#pragma unroll
-      for (int a = 0; a < TM; a++)
-#pragma unroll
-        for (int b = 0; b < TN; b++) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
-    }
-  }
-  T *Cp = (T *)G.C + G.c_off + q * G.c_q;
-#pragma unroll
-  for (int a = 0; a < TM; a++) {
-    const int gm = m0 + row(a);
-    if (gm >= G.M) continue;
-#pragma unroll
-    for (int b = 0; b < TN; b++) {
-      const int gn = n0 + col(b);
-      if (gn < G.N) Cp[G.c_m * gm + G.c_n * gn] = acc[a][b];
-    }
-  }
-}
-
-// one component's mirror-halved transform of large planes (forward: FP64 points in; inverse: FP64 points out)
-void half_gemm(Ctx *ctx, const HalfArgs &A, bool fwd, const double *in64, const int *done) {
-  SepDev *S = ctx->sep;
-  const HalfGeo G(A.n1, A.n2);
-  const KCat cat = fwd ? K_TX32 : K_TX32I;
-  const long long nin = fwd ? (long long)G.hS1 * G.hS2 * A.nplanes : (long long)A.n1 * A.n2 * A.nplanes;
-  const double pts = (double)A.n1 * A.n2 * A.nplanes;
-  if (fwd) TDGL_LAUNCH(ctx, cat, 12.0 * pts, k_half_in<true>, nblk(nin, 256), 256, 0, A, S->hx, S->hx_ps, in64, done);
-  else TDGL_LAUNCH(ctx, cat, 8.0 * pts, k_half_in<false>, nblk(nin, 256), 256, 0, A, S->hx, S->hx_ps, nullptr, done);
-  const float *W1[2] = {A.W1, A.W1 + (size_t)G.hS1 * G.R0}, *W2[2] = {A.W2, A.W2 + (size_t)G.hS2 * G.C0};
-  const int h1[2] = {G.hS1, G.hD1}, R[2] = {G.R0, G.R1}, h2[2] = {G.hS2, G.hD2}, Cw[2] = {G.C0, G.C1};
-  for (int a = 0; a < 2; a++) {   // row product of class a: O1(r, c) = Σ_i W1a[i][r] X(off_a + i, c)
-    if (h1[a] < 1) continue;
-    BGemm B;
-    B.A = W1[a]; B.a_off = 0; B.a_q = 0; B.a_m = 1; B.a_k = R[a];
-    B.B = S->hx; B.b_off = a ? G.hS1 : 0; B.b_q = S->hx_ps; B.b_k = 1; B.b_n = A.n1;
-    B.C = S->ho; B.c_off = a ? G.R0 : 0; B.c_q = S->ho_ps; B.c_m = 1; B.c_n = G.JP;
-    B.M = h1[a]; B.N = A.n2; B.K = h1[a];
-    B.done = done;
-    dim3 g((B.M + 47) / 48, (B.N + 95) / 96, A.nplanes);
-    TDGL_LAUNCH(ctx, cat, 8.0 * pts / 2, (k_bgemm_t<48, 96, 6, 8, float>), g, 96, 0, B);
-  }
-  for (int b = 0; b < 2; b++) {   // column product of class b: O2(r, C_off + c) = Σ_k O1(r, off_b + k) W2b[k][c]
-    if (h2[b] < 1) continue;
-    BGemm B;
-    B.A = S->ho; B.a_off = (long long)G.JP * (b ? G.hS2 : 0); B.a_q = S->ho_ps; B.a_m = 1; B.a_k = G.JP;
-    B.B = W2[b]; B.b_off = 0; B.b_q = 0; B.b_k = Cw[b]; B.b_n = 1;
-    B.C = S->hx; B.c_off = (long long)G.JP * (b ? G.C0 : 0); B.c_q = S->hx_ps; B.c_m = 1; B.c_n = G.JP;
-    B.M = G.JP; B.N = h2[b]; B.K = h2[b];
-    B.done = done;
-    dim3 g((B.M + 95) / 96, (B.N + 47) / 48, A.nplanes);
-    TDGL_LAUNCH(ctx, cat, 8.0 * pts / 2, (k_bgemm_t<96, 48, 8, 6, float>), g, 96, 0, B);
-  }
-  const long long nout = fwd ? (long long)A.n1 * A.n2 * A.nplanes : (long long)G.hS1 * G.hS2 * A.nplanes;
-  if (fwd) TDGL_LAUNCH(ctx, cat, 8.0 * pts, k_half_out<true>, nblk(nout, 256), 256, 0, A, S->hx, S->hx_ps, done);
-  else TDGL_LAUNCH(ctx, cat, 12.0 * pts, k_half_out<false>, nblk(nout, 256), 256, 0, A, S->hx, S->hx_ps, done);
-}
-
 template <class TIn, class TOut, class T>
 void plane(Ctx *ctx, PlaneMulti M) {
   const int cat = sizeof(T) == 8 ? K_TX64 : K_TX32;
@@ -1397,7 +1197,7 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
     A.done = done;
   };
   if constexpr (sizeof(T) == 4) {
-    if (r32) {   // the mirror-halved FP32 transforms: one launch per direction for the three components
+    if (r32 || S->hw.x[0]) {   // the mirror-halved FP32 transforms: the three components of a direction together
       HalfMulti F, I;
       F.ncomp = I.ncomp = 3;
       F.done = I.done = done;
@@ -1413,7 +1213,7 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
       const int planes[3] = {nx - 1, nx, nx};
       for (int c = 0; c < 3; c++) {
         HalfArgs &f = F.c[c], &v = I.c[c];
-        f.in = r32[c]; f.in_base = ps; f.in_ps = ps; f.in_ld = (int)n2; f.in_j0 = 1; f.in_k0 = 1;
+        f.in = r32 ? r32[c] : nullptr; f.in_base = ps; f.in_ps = ps; f.in_ld = (int)n2; f.in_j0 = 1; f.in_k0 = 1;
         f.out = hat[c]; f.out_base = 0; f.out_ps = P; f.out_ld = ny; f.out_j0 = j0[c]; f.out_k0 = k0[c];
         f.n1 = c1[c]; f.n2 = c2[c]; f.nplanes = planes[c]; f.W1 = W1f[c]; f.W2 = W2f[c]; f.T1 = T1f[c]; f.T2 = T2f[c];
         v.in = hat[c]; v.in_base = 0; v.in_ps = P; v.in_ld = ny; v.in_j0 = j0[c]; v.in_k0 = k0[c];
@@ -1425,33 +1225,15 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
         half_tc(ctx, F, true, err);
         linesolve<T>(ctx, S, w, done);
         half_tc(ctx, I, false, err);
+      } else if (!r32) {
+        half_large(ctx, F, true, r, S->hw);
+        linesolve<T>(ctx, S, w, done);
+        half_large(ctx, I, false, nullptr, S->hw);
       } else {
         half_tx(ctx, F, true);
         linesolve<T>(ctx, S, w, done);
         half_tx(ctx, I, false);
       }
-      return;
-    }
-    if (S->hx) {   // planes too large for one block: the same mirror-halved transforms as batched products
-      const float *W1f[3] = {b[1].HVf, b[1].HUf, b[1].HVf}, *W2f[3] = {b[2].HVf, b[2].HVf, b[2].HUf};
-      const float *W1i[3] = {b[1].HVi, b[1].HUi, b[1].HVi}, *W2i[3] = {b[2].HVi, b[2].HVi, b[2].HUi};
-      T *hat[3] = {w.Xh, w.Yh, w.Zh};
-      const int c1[3] = {ny, ny - 1, ny}, c2[3] = {nz, nz, nz - 1}, j0[3] = {0, 1, 0}, k0[3] = {0, 0, 1};
-      const int planes[3] = {nx - 1, nx, nx};
-      HalfArgs f[3], v[3];
-      for (int c = 0; c < 3; c++) {
-        f[c] = HalfArgs();
-        f[c].in = nullptr; f[c].in_base = ps; f[c].in_ps = ps; f[c].in_ld = (int)n2; f[c].in_j0 = 1; f[c].in_k0 = 1;
-        f[c].out = hat[c]; f[c].out_base = 0; f[c].out_ps = P; f[c].out_ld = ny; f[c].out_j0 = j0[c]; f[c].out_k0 = k0[c];
-        f[c].n1 = c1[c]; f[c].n2 = c2[c]; f[c].nplanes = planes[c]; f[c].W1 = W1f[c]; f[c].W2 = W2f[c];
-        v[c] = HalfArgs();
-        v[c].in = hat[c]; v[c].in_base = 0; v[c].in_ps = P; v[c].in_ld = ny; v[c].in_j0 = j0[c]; v[c].in_k0 = k0[c];
-        v[c].out = z[c]; v[c].out_base = ps; v[c].out_ps = ps; v[c].out_ld = (int)n2; v[c].out_j0 = 1; v[c].out_k0 = 1;
-        v[c].n1 = c1[c]; v[c].n2 = c2[c]; v[c].nplanes = planes[c]; v[c].W1 = W1i[c]; v[c].W2 = W2i[c];
-      }
-      for (int c = 0; c < 3; c++) half_gemm(ctx, f[c], true, r[c], done);
-      linesolve<T>(ctx, S, w, done);
-      for (int c = 0; c < 3; c++) half_gemm(ctx, v[c], false, nullptr, done);
       return;
     }
   }
@@ -1686,15 +1468,14 @@ int sep_create(Ctx *ctx) {
       if ((rc = dalloc(ctx, &S->r32[c], g.d.n()))) return rc;
   // planes too large for the one-block transform take the batched products through a buffer of the first product;
   // the FP32 preconditioner's mirror-halved ones (when the one-block mirror-halved kernel does not take the planes)
-  // through its X / O2 and O1 buffers
+  // through the buffers of half_large
   const bool large = plane_smem<double>(S->ny, S->nz, S->nz) > GB_ONEBLOCK || plane_smem<float>(S->ny, S->nz, S->nz) > GB_ONEBLOCK;
   if (large && (rc = dalloc(ctx, (double **)&S->gtmp, (size_t)S->nx * S->ny * S->nz))) return rc;
   if (large && f32 && !S->tc && !half_fits(S->ny, S->nz)) {
-    const HalfGeo G(S->ny, S->nz);   // the largest component's planes (y and z extents ny, nz)
-    S->hx_ps = std::max((long long)S->ny * S->nz, (long long)G.JP * (G.C0 + G.C1));
-    S->ho_ps = (long long)G.JP * S->nz;
-    if ((rc = dalloc(ctx, &S->hx, (size_t)S->nx * S->hx_ps)) || (rc = dalloc(ctx, &S->ho, (size_t)S->nx * S->ho_ps)))
-      return rc;
+    S->hw = half_work(S->ny, S->nz);
+    for (int c = 0; c < 3; c++)
+      if ((rc = dalloc(ctx, &S->hw.x[c], (size_t)S->nx * S->hw.x_ps)) || (rc = dalloc(ctx, &S->hw.o[c], (size_t)S->nx * S->hw.o_ps)))
+        return rc;
   }
   factor_lines(ctx, S, S->wd);
   // shared memory of the plane transforms (the forward shape nj = ny, nk = nz is the largest)

@@ -11,6 +11,26 @@ namespace tdgl {
 __host__ __device__ inline int rup8(int n) { return (n + 7) & ~7; }
 __host__ __device__ inline int rup16(int n) { return (n + 15) & ~15; }
 
+const int P32_KPAD = 52;   // row length of k_half32's X
+__host__ __device__ inline int p32_ks(int KO) { return 4 * ((KO / 4) | 1); }
+
+// The class geometry of a mirror-halved transform of n1 × n2 planes: hS = ⌈n/2⌉ even and hD = ⌊n/2⌋ odd modes per
+// axis, padded to 8 (R along y, C along z).
+struct HalfGeo {
+  int hS1, hD1, hS2, hD2, R0, R1, C0, C1, JP, KP, KS, XR;
+  __host__ __device__ HalfGeo(int n1, int n2) {
+    hS1 = (n1 + 1) / 2; hD1 = n1 / 2; hS2 = (n2 + 1) / 2; hD2 = n2 / 2;
+    R0 = rup8(hS1); R1 = rup8(hD1); C0 = rup8(hS2); C1 = rup8(hD2);
+    JP = R0 + R1; KP = rup8(n2); KS = p32_ks(C0 + C1); XR = n1 > JP ? n1 : JP;
+  }
+  __host__ __device__ size_t wfloats() const {
+    return (size_t)hS1 * R0 + (size_t)hD1 * R1 + (size_t)hS2 * C0 + (size_t)hD2 * C1;
+  }
+  __host__ __device__ size_t slot(int n1, int n2) const {   // one plane's XO, O1 and Stg, rounded to 16 bytes
+    return ((size_t)XR * P32_KPAD + (size_t)KP * JP + (size_t)n1 * n2 + 3) & ~(size_t)3;
+  }
+};
+
 // One component's planes for a mirror-halved transform: plane q of the input is in[in_base + q·in_ps + (in_j0 + j)
 // + in_ld·(in_k0 + k)] (j < n1, k < n2), likewise the output.
 struct HalfArgs {
@@ -33,6 +53,15 @@ struct HalfMulti {
   int dot;                     // inverse only: fold r·z and r·z_old (DotFuse) over the written points
   DotFuse df;
 };
+
+// The same transforms for planes too large for one block (sep_half.cu): a direction of the three components through X /
+// O2 and O1 buffers per component; in64: the FP64 points of the forward direction.
+struct HalfWork {
+  float *x[3] = {nullptr, nullptr, nullptr}, *o[3] = {nullptr, nullptr, nullptr};
+  long long x_ps = 0, o_ps = 0;   // plane strides
+};
+HalfWork half_work(int ny, int nz);
+void half_large(Ctx *ctx, const HalfMulti &M, bool fwd, const double *const *in64, const HalfWork &w);
 
 // Tensor-core operand images of the mirror half blocks of a basis B(p, m) (point p, mode m) with np points:
 // E = B(p, 2m) for p, m < hS = ⌈np/2⌉ and O = B(p, 2m+1) for p, m < hD = ⌊np/2⌋.  Four images [class a][hi, lo],
