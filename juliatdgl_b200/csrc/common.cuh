@@ -232,6 +232,7 @@ struct Ctx {
   cd *W = nullptr, *W2 = nullptr, *L[3] = {}, *Rl[3] = {};
   double *Th = nullptr;   // the heat model's temperature field (node-shaped; terms.jl)
   double *Th2 = nullptr;  // with D_T per material: the field of the step before (the Jacobi update)
+  double *heat_Q = nullptr, *heat_S = nullptr, *heat_prev = nullptr;   // the sweep's old θ, sources and last planes (heat.cu)
   HeatMat hm;             // with materials: each material's Γ, γ̃, σn and D_T for the heat step
   double *drag_c = nullptr, *drag_nu = nullptr;   // the interband drag's tables ([MAXB][MAXB][3], [MAXB][MAXB])
   double *Om = nullptr, *Oms = nullptr, *Rr[3] = {};   // Oms: the copy of the frame-rate smoothing (noise)

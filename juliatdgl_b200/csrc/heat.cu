@@ -3,18 +3,30 @@
 // The reference updates θ in place in lexicographic order: a node reads the new θ of its i−1, j−1 and k−1
 // neighbours and the old θ of i+1, j+1 and k+1.  The same order on the device is a sweep over the planes
 // i + j + k = s: every node of a plane depends only on the planes before it, so each plane's nodes are updated at
-// once and the result is the reference's to the bit.  One block takes the whole sweep (the faces first, then the
-// planes, a block barrier between them): the heat model is an optional term that no benchmark configuration uses,
-// and the sweep's planes are too small to fill the GPU.
+// once and the result is the reference's to the bit.
+//
+// The sweep is a chain of nx + ny + nz planes, so all that does not depend on the new θ is done before it by the whole
+// GPU (k_heat_source): the dissipation, and the old θ and the source copied to arrays ordered by plane, where a
+// plane's columns (j, k) are consecutive.  One block then takes the planes (k_heat_sweep), the new θ of the plane
+// before in shared memory, and k_heat_store brings the result back.  What bounds the sweep is the latency of a plane:
+// a block barrier, a shared load and the FP64 chain with a division.  When one block also computed the sources and
+// read the grid's own arrays (a sector per thread and load), the heat model took 574 µs of a 683 µs step on 96×48×8
+// cells; a step there takes 226 µs now.
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 
 namespace tdgl {
 namespace {
 
-const int HT_THREADS = 1024;
+const int HT_THREADS = 1024, HT_BS = 256;
+const size_t HT_SMEM = 200 * 1024;   // shared memory for the last two planes
 
 struct HeatArgs {
   double *T;
+  double *Q, *S;        // by plane: the old θ (then the new one) and the source, [s − s0][column] (one D_T)
+  double *prev;         // the last two planes' new θ when they do not fit shared memory (2 × columns)
   BandPtrs G, F;
   const double *th[3], *ph[3], *f;
   int N, x1, x2, y1, y2, z1, z2;
@@ -65,96 +77,128 @@ __device__ __forceinline__ double band_heat(double Gam, double gk, cd g, cd f, d
   return (Gam / sqrt(1 + g2 * cabs2(g))) * ((cabs2(d) + g2 * (r * r)) * invdt2);
 }
 
-__global__ void __launch_bounds__(HT_THREADS) k_heat(HeatArgs A) {
+// the heat released at the inner node o = (i, j, k): η((dissipation + σn|E|²) + the fluids' share), terms.jl:85-110
+__device__ double heat_source(const HeatArgs &A, int i, long long o) {
   const Dim d = A.d;
-  double *T = A.T;
-  const int tid = threadIdx.x;
-  auto at = [&](int i, int j, int k) { return d.at(i, j, k); };
-  // the faces, copied from inside: x, then y (over the x faces too), then z (terms.jl:70-78)
-  const int ny1 = A.y2 + 2 - A.y1, nz1 = A.z2 + 2 - A.z1, nx1 = A.x2 + 2 - A.x1;
-  for (int t = tid; t < ny1 * nz1; t += HT_THREADS) {
-    const int j = A.y1 + t % ny1, k = A.z1 + t / ny1;
-    T[at(A.x1, j, k)] = T[at(A.x1 + 1, j, k)];
-    T[at(A.x2 + 1, j, k)] = T[at(A.x2, j, k)];
-  }
-  __syncthreads();
-  for (int t = tid; t < nx1 * nz1; t += HT_THREADS) {
-    const int i = A.x1 + t % nx1, k = A.z1 + t / nx1;
-    T[at(i, A.y1, k)] = T[at(i, A.y1 + 1, k)];
-    T[at(i, A.y2 + 1, k)] = T[at(i, A.y2, k)];
-  }
-  __syncthreads();
-  for (int t = tid; t < nx1 * ny1; t += HT_THREADS) {
-    const int i = A.x1 + t % nx1, j = A.y1 + t / nx1;
-    T[at(i, j, A.z1)] = T[at(i, j, A.z1 + 1)];
-    T[at(i, j, A.z2 + 1)] = T[at(i, j, A.z2)];
-  }
-  __syncthreads();
-  const double dt = A.dt, invdt2 = 1 / (dt * dt), den = 1 + dt * A.gam;
-  const double cx = invdt2 / A.dx2, cy = invdt2 / A.dy2, cz = invdt2 / A.dz2;
-  const int lo = A.x1 + A.margin, hi = A.x2 + 1 - A.margin;
-  const int ny = A.y2 - A.y1, nz = A.z2 - A.z1;   // interior rows and columns
   const long long sx = 1, sy = d.n1, sz = (long long)d.n1 * d.n2;
-  const double *R = A.uni ? T : A.R;
-  if (!A.uni) {   // the field of the step before, faces included
-    for (long long t = tid; t < d.n(); t += HT_THREADS) A.R[t] = T[t];
-    __syncthreads();
+  const double invdt2 = 1 / (A.dt * A.dt);
+  const double cx = invdt2 / A.dx2, cy = invdt2 / A.dy2, cz = invdt2 / A.dz2;
+  const int m = A.mat ? A.mat[o] - 1 : 0;
+  const bool in = A.x1 + A.margin < i && i < A.x2 + 1 - A.margin;
+  double src = 0.0;
+  if (in) {
+    if (A.mat) {
+      for (int mu = 0; mu < A.N; mu++) src += band_heat(A.Gm[m][mu], A.gkm[m][mu], A.G.p[mu][o], A.F.p[mu][o], invdt2);
+    } else {
+      src = band_heat(A.Gam[0], A.gk[0], A.G.p[0][o], A.F.p[0][o], invdt2);
+      for (int mu = 1; mu < A.N; mu++) src += band_heat(A.Gam[mu], A.gk[mu], A.G.p[mu][o], A.F.p[mu][o], invdt2);
+    }
   }
-  auto hm = [](double a, double b) { return a == b ? a : 2 * a * b / (a + b); };
-  // one D_T: the planes i + j + k = s in order (the in-place lexicographic sweep's bits); D_T per material: every node
-  // from R at once (the planes are then only an order of work)
-  for (int s = (A.x1 + 1) + (A.y1 + 1) + (A.z1 + 1); s <= A.x2 + A.y2 + A.z2; s++) {
-    for (int t = tid; t < ny * nz; t += HT_THREADS) {
-      const int j = A.y1 + 1 + t % ny, k = A.z1 + 1 + t / ny, i = s - j - k;
-      if (i <= A.x1 || i > A.x2) continue;
-      const long long o = at(i, j, k);
-      const double q = R[o];
-      const int m = A.mat ? A.mat[o] - 1 : 0;
-      double flux;
-      if (A.uni) {
-        flux = A.DT * (((T[o + sx] - 2 * q) + T[o - sx]) / A.dx2 + ((T[o + sy] - 2 * q) + T[o - sy]) / A.dy2 +
-                       ((T[o + sz] - 2 * q) + T[o - sz]) / A.dz2);
-      } else {
-        const double d0 = A.DTm[m];
-        auto dn = [&](long long on) { return hm(d0, A.DTm[A.mat[on] - 1]); };
-        flux = (dn(o + sx) * (R[o + sx] - q) + dn(o - sx) * (R[o - sx] - q)) / A.dx2 +
-               (dn(o + sy) * (R[o + sy] - q) + dn(o - sy) * (R[o - sy] - q)) / A.dy2 +
-               (dn(o + sz) * (R[o + sz] - q) + dn(o - sz) * (R[o - sz] - q)) / A.dz2;
-      }
-      const bool in = lo < i && i < hi;
-      double src = 0.0;
-      if (in) {
-        if (A.mat) {
-          for (int mu = 0; mu < A.N; mu++) src += band_heat(A.Gm[m][mu], A.gkm[m][mu], A.G.p[mu][o], A.F.p[mu][o], invdt2);
-        } else {
-          src = band_heat(A.Gam[0], A.gk[0], A.G.p[0][o], A.F.p[0][o], invdt2);
-          for (int mu = 1; mu < A.N; mu++) src += band_heat(A.Gam[mu], A.gk[mu], A.G.p[mu][o], A.F.p[mu][o], invdt2);
-        }
-      }
-      const double sig = A.mat ? A.sigm[m] : A.sig;
-      double acc;
-      if (A.joule) {
-        double e2 = 0.0, qj = 0.0;
-        if (in && A.f[o] > 0) {
-          if (A.qp) qj = qp_joule(A, o, sx, sy, sz);   // terms.jl:107-108
-          const double a0 = A.th[0][o - sx] - A.ph[0][o - sx], a1 = A.th[0][o] - A.ph[0][o];
-          const double b0 = A.th[1][o - sy] - A.ph[1][o - sy], b1 = A.th[1][o] - A.ph[1][o];
-          const double c0 = A.th[2][o - sz] - A.ph[2][o - sz], c1 = A.th[2][o] - A.ph[2][o];
-          const double ex = 0.5 * (a0 * a0 + a1 * a1) * cx, ey = 0.5 * (b0 * b0 + b1 * b1) * cy,
-                       ez = 0.5 * (c0 * c0 + c1 * c1) * cz;
-          e2 = (ex + ey) + ez;
-        }
-        acc = q + dt * (flux + A.eta * ((src + sig * e2) + qj));
-      } else {
-        acc = q + dt * (flux + A.eta * src);
-      }
-      double tn = (acc + dt * A.gam * A.thb) / den;
-      if (tn < 0) tn = 0.0;
-      else if (tn > A.cap) tn = A.cap;
-      T[o] = tn;
+  if (!A.joule) return A.eta * src;
+  const double sig = A.mat ? A.sigm[m] : A.sig;
+  double e2 = 0.0, qj = 0.0;
+  if (in && A.f[o] > 0) {
+    if (A.qp) qj = qp_joule(A, o, sx, sy, sz);   // terms.jl:107-108
+    const double a0 = A.th[0][o - sx] - A.ph[0][o - sx], a1 = A.th[0][o] - A.ph[0][o];
+    const double b0 = A.th[1][o - sy] - A.ph[1][o - sy], b1 = A.th[1][o] - A.ph[1][o];
+    const double c0 = A.th[2][o - sz] - A.ph[2][o - sz], c1 = A.th[2][o] - A.ph[2][o];
+    const double ex = 0.5 * (a0 * a0 + a1 * a1) * cx, ey = 0.5 * (b0 * b0 + b1 * b1) * cy, ez = 0.5 * (c0 * c0 + c1 * c1) * cz;
+    e2 = (ex + ey) + ez;
+  }
+  return A.eta * ((src + sig * e2) + qj);
+}
+
+// the update from the flux and the source (terms.jl:111-118)
+__device__ __forceinline__ double heat_node(const HeatArgs &A, double q, double flux, double src) {
+  const double acc = q + A.dt * (flux + src);
+  double tn = (acc + A.dt * A.gam * A.thb) / (1 + A.dt * A.gam);
+  if (tn < 0) tn = 0.0;
+  else if (tn > A.cap) tn = A.cap;
+  return tn;
+}
+
+// Every node of the block: a face takes the θ inside (copied x, then y, then z, terms.jl:70-78: each index clamped);
+// an inner node its source and old θ by plane, or, with D_T per material, a copy of the field (faces included) in R.
+__global__ void __launch_bounds__(HT_BS) k_heat_source(const __grid_constant__ HeatArgs A) {
+  const int nx1 = A.x2 + 2 - A.x1, ny1 = A.y2 + 2 - A.y1, nz1 = A.z2 + 2 - A.z1;
+  const long long t = (long long)blockIdx.x * HT_BS + threadIdx.x;
+  if (t >= (long long)nx1 * ny1 * nz1) return;
+  const unsigned u = (unsigned)t, b = u / (unsigned)nx1, c = b / (unsigned)ny1;
+  const int i = A.x1 + (int)(u - b * (unsigned)nx1), j = A.y1 + (int)(b - c * (unsigned)ny1), k = A.z1 + (int)c;
+  const int ii = min(max(i, A.x1 + 1), A.x2), jj = min(max(j, A.y1 + 1), A.y2), kk = min(max(k, A.z1 + 1), A.z2);
+  const long long o = A.d.at(i, j, k);
+  const bool face = i != ii || j != jj || k != kk;
+  const double q = A.T[A.d.at(ii, jj, kk)];   // no inner node changes here
+  if (face) A.T[o] = q;
+  if (!A.uni) A.R[o] = q;
+  if (face) return;
+  const double s = heat_source(A, i, o);
+  if (!A.uni) {
+    A.S[o] = s;
+    return;
+  }
+  const int ny = A.y2 - A.y1, nz = A.z2 - A.z1;
+  const long long w = (long long)((i - A.x1 - 1) + (j - A.y1 - 1) + (k - A.z1 - 1)) * (ny * nz) + (j - A.y1 - 1) + ny * (k - A.z1 - 1);
+  A.Q[w] = q;
+  A.S[w] = s;
+}
+
+// One D_T: the planes in order.  Column (j, k) of plane s holds i = s − j − k, so the old θ of i+1, j+1 and k+1 are in
+// plane s + 1 (columns c, c + 1, c + ny) and the new θ of i−1, j−1 and k−1 in plane s − 1 (c, c − 1, c − ny); beyond
+// the block's inner nodes each is the node's own old θ (the face's copy).  P2: the squared spacings are powers of two,
+// so a product by the reciprocal is the quotient's bits and the chain holds one division instead of two.
+template <bool P2>
+__global__ void __launch_bounds__(HT_THREADS) k_heat_sweep(const __grid_constant__ HeatArgs A) {
+  extern __shared__ double hsh[];
+  const int nx = A.x2 - A.x1, ny = A.y2 - A.y1, nz = A.z2 - A.z1, nc = ny * nz;   // inner nodes and columns
+  double *buf = A.prev ? A.prev : hsh;
+  const double rx = 1 / A.dx2, ry = 1 / A.dy2, rz = 1 / A.dz2;
+  auto div = [](double v, double d, double r) { return P2 ? v * r : v / d; };
+  const int ns = nx + ny + nz - 2;
+  for (int s = 0; s < ns; s++) {
+    const double *pv = buf + ((s + 1) & 1) * nc;
+    double *nw = buf + (s & 1) * nc;
+    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+      const int k = c / ny, j = c - k * ny, i = s - j - k;
+      if (i < 0 || i >= nx) continue;
+      double *Qs = A.Q + (long long)s * nc + c;
+      const double *Qn = Qs + nc;
+      const double q = Qs[0];
+      const double xp = i + 1 < nx ? Qn[0] : q, yp = j + 1 < ny ? Qn[1] : q, zp = k + 1 < nz ? Qn[ny] : q;
+      const double src = A.S[(long long)s * nc + c];
+      const double xm = i > 0 ? pv[c] : q, ym = j > 0 ? pv[c - 1] : q, zm = k > 0 ? pv[c - ny] : q;
+      const double flux = A.DT * (div((xp - 2 * q) + xm, A.dx2, rx) + div((yp - 2 * q) + ym, A.dy2, ry) + div((zp - 2 * q) + zm, A.dz2, rz));
+      const double tn = heat_node(A, q, flux, src);
+      nw[c] = tn;
+      Qs[0] = tn;
     }
     __syncthreads();
   }
+}
+
+// the inner nodes' new θ from the planes (one D_T), or from the field of the step before at once (D_T per material)
+__global__ void __launch_bounds__(HT_BS) k_heat_store(const __grid_constant__ HeatArgs A) {
+  const int nx = A.x2 - A.x1, ny = A.y2 - A.y1, nz = A.z2 - A.z1;
+  const long long t = (long long)blockIdx.x * HT_BS + threadIdx.x;
+  if (t >= (long long)nx * ny * nz) return;
+  const unsigned u = (unsigned)t, b = u / (unsigned)nx, k = b / (unsigned)ny;
+  const int i = (int)(u - b * (unsigned)nx), j = (int)(b - k * (unsigned)ny);
+  const long long o = A.d.at(A.x1 + 1 + i, A.y1 + 1 + j, A.z1 + 1 + (int)k);
+  if (A.uni) {
+    A.T[o] = A.Q[(long long)(i + j + (int)k) * (ny * nz) + j + ny * (int)k];
+    return;
+  }
+  const long long sx = 1, sy = A.d.n1, sz = (long long)A.d.n1 * A.d.n2;
+  const double *R = A.R;
+  const double q = R[o], d0 = A.DTm[A.mat[o] - 1];
+  auto dn = [&](long long on) {
+    const double e = A.DTm[A.mat[on] - 1];
+    return d0 == e ? d0 : 2 * d0 * e / (d0 + e);
+  };
+  const double flux = (dn(o + sx) * (R[o + sx] - q) + dn(o - sx) * (R[o - sx] - q)) / A.dx2 +
+                      (dn(o + sy) * (R[o + sy] - q) + dn(o - sy) * (R[o - sy] - q)) / A.dy2 +
+                      (dn(o + sz) * (R[o + sz] - q) + dn(o - sz) * (R[o - sz] - q)) / A.dz2;
+  A.T[o] = heat_node(A, q, flux, A.S[o]);
 }
 
 __global__ void k_fill(double *a, double v, long long n) {
@@ -183,6 +227,16 @@ int heat_create(Ctx *ctx, const tdgl_materials *M) {
     }
     if (!uni && (rc = dalloc(ctx, &ctx->Th2, (size_t)nn))) return rc;
   }
+  // the source (with D_T per material by node, else by plane beside the old θ), and the last two planes' θ where they do
+  // not fit shared memory
+  const Geo &g = ctx->g;
+  const size_t nc = (size_t)std::max(1, g.y2 - g.y1) * std::max(1, g.z2 - g.z1);
+  const size_t np = (size_t)std::max(1, (g.x2 - g.x1) + (g.y2 - g.y1) + (g.z2 - g.z1) - 2) * nc;
+  if ((rc = dalloc(ctx, &ctx->heat_S, ctx->Th2 ? (size_t)nn : np))) return rc;
+  if (!ctx->Th2 && (rc = dalloc(ctx, &ctx->heat_Q, np))) return rc;
+  if (!ctx->Th2 && 2 * nc * sizeof(double) > HT_SMEM && (rc = dalloc(ctx, &ctx->heat_prev, 2 * nc))) return rc;
+  smem_optin(k_heat_sweep<false>);
+  smem_optin(k_heat_sweep<true>);
   TDGL_LAUNCH(ctx, K_HEAT, 8.0 * nn, k_fill, nblk(nn, 256), 256, 0, ctx->Th, ctx->P.heat_T, nn);
   return 0;
 }
@@ -217,6 +271,9 @@ void heat_step(Ctx *ctx) {
   A.mat = ctx->mat;
   A.uni = ctx->Th2 == nullptr;
   A.R = ctx->Th2;
+  A.Q = ctx->heat_Q;
+  A.S = ctx->heat_S;
+  A.prev = ctx->heat_prev;
   A.qp = P.qp_on;
   qp_potentials(ctx, A.qmu);
   A.qsig = P.qp_sigma_n;
@@ -232,8 +289,21 @@ void heat_step(Ctx *ctx) {
     A.sigm[m] = ctx->hm.sig[m];
     A.DTm[m] = ctx->hm.DT[m];
   }
-  const double n = (double)(g.x2 - g.x1) * (g.y2 - g.y1) * (g.z2 - g.z1);
-  TDGL_LAUNCH(ctx, K_HEAT, n * (8.0 * 8 + 32.0 * ctx->N), k_heat, 1, HT_THREADS, 0, A);
+  const long long ni = (long long)(g.x2 - g.x1) * (g.y2 - g.y1) * (g.z2 - g.z1), nc = (long long)(g.y2 - g.y1) * (g.z2 - g.z1);
+  const long long nb = (long long)(g.x2 + 2 - g.x1) * (g.y2 + 2 - g.y1) * (g.z2 + 2 - g.z1);
+  TDGL_LAUNCH(ctx, K_HEAT, nb * (8.0 * 9 + 32.0 * ctx->N), k_heat_source, nblk(nb, HT_BS), HT_BS, 0, A);
+  if (ni <= 0) return;
+  if (A.uni) {
+    auto pow2 = [](double v) {
+      int e;
+      return std::frexp(v, &e) == 0.5 && std::isnormal(1 / v);
+    };
+    const int threads = (int)std::min<long long>(HT_THREADS, (nc + 31) / 32 * 32);
+    const size_t smem = A.prev ? 0 : 2 * nc * sizeof(double);
+    if (pow2(A.dx2) && pow2(A.dy2) && pow2(A.dz2)) TDGL_LAUNCH(ctx, K_HEAT, 32.0 * ni, k_heat_sweep<true>, 1, threads, smem, A);
+    else TDGL_LAUNCH(ctx, K_HEAT, 32.0 * ni, k_heat_sweep<false>, 1, threads, smem, A);
+  }
+  TDGL_LAUNCH(ctx, K_HEAT, 16.0 * ni, k_heat_store, nblk(ni, HT_BS), HT_BS, 0, A);
 }
 
 int heat_carry(Ctx *ctx, double *host, bool up) {
