@@ -119,8 +119,8 @@ __device__ __forceinline__ void scale_b(const Blk bk, ScaleArgs const &A) {
 // What bounds it: an FP64 sincos per link on large grids; on small ones it is one launch where the links with the
 // curl, the faces of h, the ghosts of each band and the copy of advance! were N + 3, each waiting for the one before.
 // 40 steps took 2709 µs instead of 2811 (12×8×4 cells), 3597 instead of 3782 (64×32×8), 7638 instead of 7893
-// (192×64×16), 245.9 ms instead of 250.0 (the 256×128×32 ramp).  The ghosts are a call, not inlined, and the registers
-// are held to 32: inlined (110 registers) the links lost their occupancy and the 192×64×16 cycle took 8252 µs.
+// (192×64×16), 245.9 ms instead of 250.0 (the 256×128×32 ramp).  The registers are held to 40: with the
+// ghosts' sincos inlined three times (110 registers) the links lost their occupancy and the 192×64×16 cycle took 8252 µs.
 struct FinArgs {
   const double *ph[3];
   cd *U[3];
@@ -270,30 +270,38 @@ __device__ __forceinline__ void face_point(const FinArgs &A, int comp, int i, in
   A.h[comp][o] = v;
 }
 
-// The three face passes of ghosts! (bands.jl:524-539) at a point of the block's shell: the writes that reach it in the
-// reference's order (x faces, then y, then z).  A z-face point takes the z pass over the value the y or x pass left at
-// z1+1 / z2, a y-face point (k inside) the y pass over the x pass's value, an x-face point (j, k inside) the x pass.
-__device__ __noinline__ cd ghost_point(const FinArgs &A, const cd *X, int i, int j, int k) {
+// The three face passes of ghosts! (bands.jl:524-539) at the point o = (i, j, k) of the block's shell, every band: the
+// writes that reach it in the reference's order (x faces, then y, then z).  An x-face point takes the x pass's link
+// times the node inside; a y-face point the y pass over that (at the first column inside), a z-face point the z pass
+// over both (at the first plane inside).  One pass at a time, through F[o], each link formed once for all bands by a
+// single sincos site: the chain of up to three per band made the launch 9 µs on 12×8×4 cells (its cycle went from 2160
+// to 1990 µs), and the kernel stays at 40 registers.
+__device__ __forceinline__ void ghost_point(const FinArgs &A, int i, int j, int k, long long o) {
   const Dim d = A.d;
-  const int x1 = A.x1, x2 = A.x2, y1 = A.y1, y2 = A.y2, z1 = A.z1, z2 = A.z2;
-  auto lk = [&](int ax, long long q) { return ccis(-A.ph[ax][q]); };
-  auto after_x = [&](int i, int j, int k) -> cd {
-    if (i == x1) return cmul(lk(0, d.at(x1, j, k)), X[d.at(x1 + 1, j, k)]);
-    if (i == x2 + 1) return cmul(cconj(lk(0, d.at(x2, j, k))), X[d.at(x2, j, k)]);
-    return X[d.at(i, j, k)];
-  };
-  auto after_y = [&](int i, int j, int k) -> cd {
-    if (j == y1) return cmul(lk(1, d.at(i, y1, k)), after_x(i, y1 + 1, k));
-    if (j == y2 + 1) return cmul(cconj(lk(1, d.at(i, y2, k))), after_x(i, y2, k));
-    return after_x(i, j, k);
-  };
-  if (k == z1) return cmul(lk(2, d.at(i, j, z1)), after_y(i, j, z1 + 1));
-  if (k == z2 + 1) return cmul(cconj(lk(2, d.at(i, j, z2))), after_y(i, j, z2));
-  return after_y(i, j, k);
+  const int ii = min(max(i, A.x1 + 1), A.x2), jj = min(max(j, A.y1 + 1), A.y2), kk = min(max(k, A.z1 + 1), A.z2);
+  long long src = d.at(ii, jj, kk);   // the node inside, then the pass before
+#pragma unroll 1
+  for (int ax = 0; ax < 3; ax++) {
+    const int at = ax == 0 ? i : ax == 1 ? j : k, lo = ax == 0 ? A.x1 : ax == 1 ? A.y1 : A.z1;
+    const int hi = ax == 0 ? A.x2 : ax == 1 ? A.y2 : A.z2;
+    if (at != lo && at != hi + 1) continue;
+    const int e = at == lo ? lo : hi;   // the link along ax that ends on the face
+    const long long q = ax == 0 ? d.at(e, jj, kk) : ax == 1 ? d.at(i, e, kk) : d.at(i, j, e);
+    cd u = ccis(-A.ph[ax][q]);
+    if (at != lo) u = cconj(u);
+    for (int mu = 0; mu < A.N; mu++) A.F[mu][o] = cmul(u, A.F[mu][src]);
+    src = o;
+  }
+  const bool vac = A.vac && A.vac[o];
+  for (int mu = 0; mu < A.N; mu++) {
+    const cd v = vac ? mkc(0.0, 0.0) : A.F[mu][o];
+    if (vac) A.F[mu][o] = v;
+    A.G[mu][o] = v;
+  }
 }
 
 __device__ __forceinline__ void finish_b(const Blk bk, FinArgs const &A);
-__global__ void __launch_bounds__(BS, 8) k_finish(const __grid_constant__ FinArgs A) { finish_b(TDGL_BLK, A); }
+__global__ void __launch_bounds__(BS, 6) k_finish(const __grid_constant__ FinArgs A) { finish_b(TDGL_BLK, A); }
 TDGL_MERGEABLE(k_finish, finish_b, BS, 6, false);
 __device__ __forceinline__ void finish_b(const Blk bk, FinArgs const &A) {
   long long t = (long long)bk.x * blockDim.x + threadIdx.x;
@@ -328,15 +336,14 @@ __device__ __forceinline__ void finish_b(const Blk bk, FinArgs const &A) {
   } else {
     const bool block = i >= A.x1 && i <= A.x2 + 1 && j >= A.y1 && j <= A.y2 + 1 && k >= A.z1 && k <= A.z2 + 1;
     const bool shell = i == A.x1 || i == A.x2 + 1 || j == A.y1 || j == A.y2 + 1 || k == A.z1 || k == A.z2 + 1;
+    if (block && shell) {
+      ghost_point(A, i, j, k, o);
+      return;
+    }
     const bool vac = A.vac && A.vac[o];
     for (int mu = 0; mu < A.N; mu++) {
-      if (!block) {   // with vacuum only
-        if (vac) A.F[mu][o] = mkc(0.0, 0.0);
-        continue;
-      }
-      const cd v = vac ? mkc(0.0, 0.0) : shell ? ghost_point(A, A.F[mu], i, j, k) : A.F[mu][o];
-      if (shell || vac) A.F[mu][o] = v;
-      A.G[mu][o] = v;
+      if (vac) A.F[mu][o] = mkc(0.0, 0.0);
+      if (block) A.G[mu][o] = vac ? mkc(0.0, 0.0) : A.F[mu][o];   // outside the block: with vacuum only
     }
   }
 }
