@@ -1315,23 +1315,26 @@ int tdgl_sep_apply(tdgl_ctx *c, const double *b, double *z, int32_t f32) {
   // packed host ranges → plane-major device arrays → solve → back (through the PCG carry helpers' layout)
   const long long nn = ctx->g.d.n();
   double *d[3] = {nullptr, nullptr, nullptr};
+  float *f[3] = {nullptr, nullptr, nullptr};   // the FP32 preconditioner's z
   cudaError_t e = cudaSuccess;
   for (int q = 0; q < 3 && e == cudaSuccess; q++) {
     e = cudaMalloc(&d[q], nn * sizeof(double));
     if (e == cudaSuccess) e = cudaMemsetAsync(d[q], 0, nn * sizeof(double), ctx->stream);
+    if (e == cudaSuccess && f32) e = cudaMalloc(&f[q], nn * sizeof(float));
+    if (e == cudaSuccess && f32) e = cudaMemsetAsync(f[q], 0, nn * sizeof(float), ctx->stream);
   }
-  if (e == cudaSuccess) {
-    int rc = pm_from_packed_host(ctx, d, b);
-    if (!rc) {
-      sep_apply(ctx, d, d, f32 != 0, nullptr);
-      rc = pm_to_packed_host(ctx, d, z);
-    }
-    for (int q = 0; q < 3; q++) cudaFree(d[q]);
-    return rc;
+  int rc = e == cudaSuccess ? 0 : set_err(ctx, TDGL_ECUDA, "sep_apply", e);
+  if (!rc) rc = pm_from_packed_host(ctx, d, b);
+  if (!rc) {
+    sep_apply(ctx, d, f32 ? (void *const *)f : (void *const *)d, f32 != 0, nullptr);
+    for (int q = 0; q < 3 && f32; q++) sep_widen(ctx, f[q], d[q], nn);
+    rc = pm_to_packed_host(ctx, d, z);
   }
-  for (int q = 0; q < 3; q++)
+  for (int q = 0; q < 3; q++) {
     if (d[q]) cudaFree(d[q]);
-  return set_err(ctx, TDGL_ECUDA, "sep_apply", e);
+    if (f[q]) cudaFree(f[q]);
+  }
+  return rc;
 }
 
 int tdgl_profile(tdgl_ctx *c, int32_t on) {

@@ -5,9 +5,9 @@
 // warm start and the extrapolated first guess 2xₙ − xₙ₋₁ of pcg_fast (_implicit_curl_fast! :376-446), the
 // zero-source update (_pcg_zero_update! :251-271), and φ = θ + (φₑ − θ)/D on the decoupled links.
 //
-// Iterates, residuals and dot products are FP64.  Every vector is a plane-major node-shaped array per component
-// (sep.cu), zero outside the ranges, so the vector kernels are flat loops.  A·p computes the curl of p on the fly
-// (no plaquette arrays).  Dot products are deterministic: a fixed grid of block partial sums reduced by one block
+// Iterates, residuals and dot products are FP64; z is held in the precision the preconditioner computes it in.  Every
+// vector is a plane-major node-shaped array per component (sep.cu), zero outside the ranges, so the vector kernels are
+// flat loops.  A·p forms the new direction p = z + βp and the curl of p on the fly (no plaquette arrays).  Dot products are deterministic: a fixed grid of block partial sums reduced by one block
 // in a fixed order.  The loop runs on the device: α, β and the convergence test (‖r‖ ≤ tol·‖b‖) are computed by
 // the reduction kernels, and once the test passes every later kernel of the iteration returns at once; the host
 // launches iterations in batches and reads the flag between batches only.
@@ -24,15 +24,16 @@ Rng sep_range(const Geo &g, int ax);
 void to_planes(Ctx *ctx, const double *const *a, const double *const *b, double *const *out);
 void from_planes(Ctx *ctx, const double *const *in, const double *const *base, double *const *out);
 
-static const int RED_BLOCKS = 740;   // at most 5 × 148 SMs (the stencil: five blocks per SM, launch bounds below)
 static const int STR_BLOCKS = 1184;  // at most 8 × 148 SMs: full occupancy for the streaming kernels
 static const int BATCH = 4;          // iterations between two reads of the convergence flag
 
 struct PcgDev {
-  double *P[3] = {}, *Q[3] = {}, *x[3] = {}, *r[3] = {}, *z[3] = {}, *b[3] = {}, *xprev[3] = {}, *zold[3] = {}, *Dp[3] = {};
-  double *part = nullptr;                       // STR_BLOCKS × 2 partial sums
-  double *part2 = nullptr;                      // xblocks partial sums of r·z_old (k_dot_part)
-  cudaStream_t side = nullptr;                  // the x update and r·z_old beside the preconditioner
+  double *P[2][3] = {}, *Q[3] = {}, *x[3] = {}, *r[3] = {}, *b[3] = {}, *xprev[3] = {}, *Dp[3] = {};
+  void *z[2][3] = {};                           // z and the z before (FP32 with the FP32 preconditioner)
+  uint8_t *Dc[3] = {};                          // σ_l/σ_n as codes into Dt (null: more than 256 values)
+  double *Dt = nullptr;
+  double *part = nullptr;                       // partial sums (two per block)
+  cudaStream_t side = nullptr;                  // the x update beside the preconditioner
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   int xblocks = 1;                              // grid of the kernels beside the preconditioner (2 per SM at most)
   double *sc = nullptr;                         // device scalars SC_*
@@ -44,7 +45,8 @@ struct PcgDev {
   long long tcwait_seen = 0;                    // ST_TCWAIT at the last status read
   bool warm = false, have2 = false;
   long long n;                                  // node count (per component array)
-  int sblocks = STR_BLOCKS, ablocks = RED_BLOCKS;   // grids of the streaming kernels and of A·p for this size
+  int sblocks = STR_BLOCKS;                     // grid of the streaming kernels for this size
+  int tj = 1, tk = 1, ntj = 1, ntk = 1, chunk = 1, nchunk = 1;   // A·p: tile, tiles along j and k, planes per block
 };
 
 namespace {
@@ -61,7 +63,12 @@ struct F3 {                  // FP32 copy of a vector (p[0] null: none)
 };
 
 // partial sums of a·b and a·c (c may be null) over the three component arrays
-__global__ void __launch_bounds__(256, 8) k_dot2(CVec3 a, CVec3 b, CVec3 c, int use_c, long long n, double *part, const int *ic, Fold F) {
+template <class T>
+struct ZVec3 {
+  const T *p[3];
+};
+template <class T>
+__global__ void __launch_bounds__(256, 8) k_dot2(CVec3 a, ZVec3<T> b, ZVec3<T> c, int use_c, long long n, double *part, const int *ic, Fold F) {
   if (ic && ic[IC_DONE]) return;
   __shared__ double sh[32];
   double s1 = 0.0, s2 = 0.0;
@@ -70,8 +77,8 @@ __global__ void __launch_bounds__(256, 8) k_dot2(CVec3 a, CVec3 b, CVec3 c, int 
 #pragma unroll 2
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
       const double av = a.p[cc][t];
-      s1 += av * b.p[cc][t];
-      if (use_c) s2 += av * c.p[cc][t];
+      s1 += av * (double)b.p[cc][t];
+      if (use_c) s2 += av * (double)c.p[cc][t];
     }
   double r1 = block_sum(s1, sh);
   __syncthreads();
@@ -85,79 +92,219 @@ __global__ void __launch_bounds__(256, 8) k_dot2(CVec3 a, CVec3 b, CVec3 c, int 
 }
 
 // Q = D P + a curl curl P on the ranges (implicit.jl:212-235), the plaquette fields computed on the fly, with the
-// partial sums of P·Q.  One thread per node of the box i ∈ 2..Nx, j ∈ 2..Ny, k ∈ 2..Nz (plane-major order; node
-// counts fit 32 bits, checked at set-up).
+// partial sums of P·Q, over the box i ∈ 2..Nx, j ∈ 2..Ny, k ∈ 2..Nz.  With DIR the direction is formed here too,
+// P = z + βP (the solve's first iteration, ic[IC_ITERS] = 0: P = z), from the old P into the other buffer.
+//
+// What bounds it: HBM.  A block takes a tile of tj × tk columns (tj ≤ 24 rows of the unit-stride axis; both split
+// evenly), a column per thread, and marches over `chunk` planes i.  A thread reads its own column (and one element of
+// the tile's halo) straight into registers two planes ahead, forms P, and leaves it in shared memory for its
+// neighbours: three planes in turn, so that one barrier a plane suffices.  The plaquettes of plane i − 1 that plane i
+// needs are the thread's own, kept in registers.  Each plane is read once per tile with a halo of one row and column.
+// The conductivities are a byte per link where they have at most 256 values (padding, materials), looked up in shared
+// memory.  One thread per node reading its 36 neighbours through L1 fetched each plane several times from L2, and the
+// direction was a pass of its own: 57 + 24 µs on the 256×128×32 ramp, 78 + 31 on 97 × 287 × 95 unknowns a component;
+// this kernel takes 48 and 61.  320 threads: with more, the registers of two blocks per SM do not hold the planes
+// ahead (352 threads: 70 µs); 24 rows: the halo of a nearly square tile is the smallest.
 struct ApplyArgs {
-  const double *P[3], *D[3];
+  const double *P[3];
+  const void *Z[3];
+  double *Pn[3];
+  const double *D[3];
+  const uint8_t *Dc[3];
+  const double *Dt;
   double *Q[3];
-  double sxy, sxz, syx, syz, szx, szy, dx, dy, dz, iyz, izx, ixy;
+  double sxy, sxz, syx, syz, szx, szy, iyz, izx, ixy;
   int Nx, Ny, Nz, n2, n3;
+  int tj, tk, ntj, ntk, chunk;
+  const double *sc;
   double *part;
   const int *ic;
+  int gated;
   Fold F;
 };
+const int AP_T = 320;
+// the tile's halo, three components of one element each, must not outnumber the threads: tj + tk ≤ AP_T / 6 − 2
+const int AP_TJ = 24, AP_SUM = AP_T / 6 - 2;
 
-__global__ void __launch_bounds__(256, 5) k_apply(ApplyArgs A) {
-  if (A.ic && A.ic[IC_DONE]) return;
+__host__ __device__ constexpr size_t apply_smem(int tj, int tk) {   // three planes of P; the conductivity table
+  return ((size_t)9 * (tj + 2) * (tk + 2) + 256) * sizeof(double);
+}
+
+// what a thread reads of a plane ahead of its use: its own column's old P and z, and its halo element's
+template <class TZ>
+struct ApRaw {
+  double p[3], hp;
+  TZ z[3], hz;
+};
+
+template <class TZ, bool DIR>
+__global__ void __launch_bounds__(AP_T, 2) k_apply(const __grid_constant__ ApplyArgs A) {
+  if (A.gated && A.ic[IC_DONE]) return;
   __shared__ double sh[32];
-  const int Nx = A.Nx, Ny = A.Ny, Nz = A.Nz;
-  const long long sj = 1, sk = A.n2, si = (long long)A.n2 * A.n3;
-  const int nj = Ny - 1, nk = Nz - 1, ni = Nx - 1;
-  // distinct arrays (P and D read, Q written): the compiler may keep several nodes' loads in flight, which this
-  // latency-bound kernel needs (the stores to Q cannot alias the loads of P)
-  const double *__restrict__ px = A.P[0], *__restrict__ py = A.P[1], *__restrict__ pz = A.P[2];
-  const double *__restrict__ Dx = A.D[0], *__restrict__ Dy = A.D[1], *__restrict__ Dz = A.D[2];
-  double *__restrict__ Qx = A.Q[0], *__restrict__ Qy = A.Q[1], *__restrict__ Qz = A.Q[2];
-  // the plaquette areas as reciprocals: nine FP64 divisions per node were half of this kernel's instructions (the
-  // operator differs from the reference's division by at most an ulp per plaquette field)
-  const double iyz = A.iyz, izx = A.izx, ixy = A.ixy;
-  auto at = [&](int i, int j, int k) { return (long long)(j - 1) + A.n2 * ((long long)(k - 1) + (long long)A.n3 * (i - 1)); };
-  auto hx = [&](int i, int j, int k) -> double {
-    if (k < 2 || k > Nz - 1 || j < 2 || j > Ny - 1 || i < 2 || i > Nx) return 0.0;
-    const long long o = at(i, j, k);
-    return ((pz[o + sj] - pz[o]) - py[o + sk] + py[o]) * iyz;
-  };
-  auto hy = [&](int i, int j, int k) -> double {
-    if (k < 2 || k > Nz - 1 || j < 2 || j > Ny || i < 2 || i > Nx - 1) return 0.0;
-    const long long o = at(i, j, k);
-    return ((px[o + sk] - px[o]) - pz[o + si] + pz[o]) * izx;
-  };
-  auto hz = [&](int i, int j, int k) -> double {
-    if (k < 2 || k > Nz || j < 2 || j > Ny - 1 || i < 2 || i > Nx - 1) return 0.0;
-    const long long o = at(i, j, k);
-    return ((py[o + si] - py[o]) - px[o + sj] + px[o]) * ixy;
-  };
-  double s = 0.0;
-  const int n = nj * nk * ni;
-#pragma unroll 2
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const int j = 2 + t % nj, u = t / nj;
-    const int k = 2 + u % nk, i = 2 + u / nk;
-    const long long o = at(i, j, k);
-    const double hx0 = hx(i, j, k), hy0 = hy(i, j, k), hz0 = hz(i, j, k);
-    if (i <= Nx - 1) {
-      const double q = Dx[o] * px[o] + A.sxy * (hz0 - hz(i, j - 1, k)) - A.sxz * (hy0 - hy(i, j, k - 1));
-      Qx[o] = q;
-      s += px[o] * q;
+  extern __shared__ __align__(16) double apsm[];
+  const int Nx = A.Nx, Ny = A.Ny, Nz = A.Nz, W = A.tj + 2, E = W * (A.tk + 2), nc = A.tj * A.tk;
+  double *const tab = apsm, *const ps = apsm + 256;     // P: [plane in turn][component][E]
+  const int tid = threadIdx.x;
+  const int bj = blockIdx.x % A.ntj, bk = (blockIdx.x / A.ntj) % A.ntk, bi = blockIdx.x / (A.ntj * A.ntk);
+  const int j0 = 2 + bj * A.tj, k0 = 2 + bk * A.tk;                 // the tile's first node
+  const int i0 = 2 + bi * A.chunk, i1 = min(Nx, i0 + A.chunk - 1);   // the block's planes
+  const int si = A.n2 * A.n3;                                        // (the context's node counts fit 32 bits)
+  const bool coded = A.Dc[0] != nullptr;
+  if (coded)
+    for (int t = tid; t < 256; t += AP_T) tab[t] = A.Dt[t];
+  const bool first = DIR && A.ic[IC_ITERS] == 0;
+  const double beta = DIR && !first ? A.sc[SC_BETA] : 0.0;
+  // this thread's column, and its halo element (a row of W below and above the tile, then the two columns beside it)
+  const int jj = 1 + tid % A.tj, kk = 1 + tid / A.tj, j = j0 - 1 + jj, k = k0 - 1 + kk;
+  const bool in = tid < nc && j <= A.n2 && k <= A.n3, act = tid < nc && j <= Ny && k <= Nz;
+  const int e0 = jj + W * kk, oc = (j - 1) + A.n2 * (k - 1);
+  const int H = E - nc, hc = tid / H, h = tid - hc * H;
+  const int hj = h < 2 * W ? h % W : (h - 2 * W) / A.tk * (A.tj + 1);
+  const int hk = h < 2 * W ? h / W * (A.tk + 1) : 1 + (h - 2 * W) % A.tk;
+  const bool ring = hc < 3, hin = ring && j0 - 1 + hj <= A.n2 && k0 - 1 + hk <= A.n3;
+  const int he = hj + W * hk, ho = (j0 + hj - 2) + A.n2 * (k0 + hk - 2);
+  const double *const hP = A.P[ring ? hc : 0];
+  const TZ *const hZ = (const TZ *)A.Z[ring ? hc : 0];
+  auto load = [&](ApRaw<TZ> &R, int i) {
+    if (i > i1 + 1) return;
+    const int pl = si * (i - 1);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      R.p[c] = in ? A.P[c][pl + oc] : 0.0;
+      if (DIR) R.z[c] = in ? ((const TZ *)A.Z[c])[pl + oc] : TZ(0);
     }
-    if (j <= Ny - 1) {
-      const double q = Dy[o] * py[o] + A.syz * (hx0 - hx(i, j, k - 1)) - A.syx * (hz0 - hz(i - 1, j, k));
-      Qy[o] = q;
-      s += py[o] * q;
+    R.hp = hin ? hP[pl + ho] : 0.0;
+    if (DIR) R.hz = hin ? hZ[pl + ho] : TZ(0);
+  };
+  auto dir = [&](double p, TZ z) { return !DIR ? p : first ? (double)z : (double)z + beta * p; };
+  // plane i from its raw values: P into v, shared memory and (the block's own planes) memory
+  auto enter = [&](const ApRaw<TZ> &R, int i, double *slot, double (&v)[3]) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) v[c] = dir(R.p[c], R.z[c]);
+    if (tid < nc) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) slot[c * E + e0] = v[c];
     }
-    if (k <= Nz - 1) {
-      const double q = Dz[o] * pz[o] + A.szx * (hy0 - hy(i - 1, j, k)) - A.szy * (hx0 - hx(i, j - 1, k));
-      Qz[o] = q;
-      s += pz[o] * q;
+    if (ring) slot[hc * E + he] = dir(R.hp, R.hz);
+    if (DIR && act && i >= i0 && i <= i1) {
+      const int o = si * (i - 1) + oc;
+#pragma unroll
+      for (int c = 0; c < 3; c++) A.Pn[c][o] = v[c];
     }
+  };
+  unsigned cd[3] = {0, 0, 0};
+  double Dv[3] = {0.0, 0.0, 0.0};
+  auto conduct = [&](int i) {   // the conductivities of plane i, a plane ahead
+    if (!act || i < i0 || i > i1) return;
+    const int o = si * (i - 1) + oc;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (coded) cd[c] = A.Dc[c][o];
+      else Dv[c] = A.D[c][o];
+    }
+  };
+  const bool ky = k <= Nz - 1, jy = j <= Ny - 1;   // plaquettes beside this node exist
+  const bool kp = k >= 3, jp = j >= 3;             // and before it
+  double hyp = 0.0, hzp = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
+  double v0[3], v1[3];
+  double *s0 = ps, *s1 = ps + 3 * E, *s2 = ps + 6 * E;
+  ApRaw<TZ> R0, R1;
+  load(R0, i0 - 1);
+  load(R1, i0);
+  enter(R0, i0 - 1, s0, v0);
+  load(R0, i0 + 1);
+  auto step = [&](int i, ApRaw<TZ> &R) {   // plane i, plane i + 1 in R
+    enter(R, i + 1, s1, v1);
+    load(R, i + 3);
+    double d[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) d[c] = coded ? 0.0 : Dv[c];
+    unsigned dc[3] = {cd[0], cd[1], cd[2]};
+    conduct(i + 1);
+    __syncthreads();   // plane i + 1 is there for all; the slot written next was last read before this barrier
+    if (act) {
+      if (coded) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) d[c] = tab[dc[c]];
+      }
+      const double *px = s0 + e0, *py = px + E, *pz = py + E, *qy = s1 + E + e0, *qz = qy + E;
+      const double x0 = v0[0], y0 = v0[1], z0 = v0[2];
+      // the plaquette areas as reciprocals: nine FP64 divisions per node were half of this kernel's instructions (the
+      // operator differs from the reference's division by at most an ulp per plaquette field)
+      double hy0 = 0.0, hz0 = 0.0;
+      if (i >= 2 && i <= Nx - 1) {
+        if (ky) hy0 = ((px[W] - x0) - v1[2] + z0) * A.izx;
+        if (jy) hz0 = ((v1[1] - y0) - px[1] + x0) * A.ixy;
+      }
+      if (i >= i0) {
+        const int o = si * (i - 1) + oc;
+        if (i <= Nx - 1) {
+          const double pm = px[-1], pw = px[-W];
+          const double hzm = jp ? ((qy[-1] - py[-1]) - x0 + pm) * A.ixy : 0.0;
+          const double hym = kp ? ((x0 - pw) - qz[-W] + pz[-W]) * A.izx : 0.0;
+          const double q = d[0] * x0 + A.sxy * (hz0 - hzm) - A.sxz * (hy0 - hym);
+          A.Q[0][o] = q;
+          sx += x0 * q;
+        }
+        const double hx0 = ky && jy ? ((pz[1] - z0) - py[W] + y0) * A.iyz : 0.0;
+        if (jy) {
+          const double hxm = kp ? ((pz[1 - W] - pz[-W]) - y0 + py[-W]) * A.iyz : 0.0;
+          const double q = d[1] * y0 + A.syz * (hx0 - hxm) - A.syx * (hz0 - hzp);
+          A.Q[1][o] = q;
+          sy += y0 * q;
+        }
+        if (ky) {
+          const double hxm = jp ? ((z0 - pz[-1]) - py[W - 1] + py[-1]) * A.iyz : 0.0;
+          const double q = d[2] * z0 + A.szx * (hy0 - hyp) - A.szy * (hx0 - hxm);
+          A.Q[2][o] = q;
+          sz += z0 * q;
+        }
+      }
+      hyp = hy0;
+      hzp = hz0;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) v0[c] = v1[c];
+    double *s = s0;
+    s0 = s1;
+    s1 = s2;
+    s2 = s;
+  };
+  for (int i = i0 - 1; i <= i1; i += 2) {
+    step(i, R1);
+    if (i + 1 <= i1) step(i + 1, R0);
   }
-  const double r = block_sum(s, sh);
-  if (threadIdx.x == 0) {
+  const double r = block_sum((sx + sy) + sz, sh);
+  if (tid == 0) {
     A.part[blockIdx.x] = r;
     A.part[gridDim.x + blockIdx.x] = 0.0;
   }
   __syncthreads();
   fold_last(A.F, A.part, sh);
+}
+
+// The distinct values of the conductivities as a table of at most 256, and each entry's place in it: an open-addressed
+// set of bit patterns (a value takes its hash's slot or a later one).  *bad counts the entries that found no place.
+const unsigned long long DT_FREE = 0xfff8dead0000beefULL;   // no value a conductivity has (a NaN with this payload)
+__global__ void k_dtab_clear(unsigned long long *tab, int *bad) {
+  tab[threadIdx.x] = DT_FREE;
+  if (threadIdx.x == 0) *bad = 0;
+}
+__global__ void k_dtab(CVec3 D, long long n, unsigned long long *tab, uint8_t *c0, uint8_t *c1, uint8_t *c2, int *bad) {
+  uint8_t *code[3] = {c0, c1, c2};
+  for (int c = 0; c < 3; c++)
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+      const unsigned long long v = (unsigned long long)__double_as_longlong(D.p[c][t]);
+      unsigned h = (unsigned)((v ^ (v >> 29) ^ (v >> 47)) * 0x9e3779b1u) >> 24;
+      int left = 256;
+      for (; left > 0; left--, h = (h + 1) & 255) {
+        unsigned long long w = *(volatile unsigned long long *)(tab + h);
+        if (w == DT_FREE) w = atomicCAS(tab + h, DT_FREE, v);
+        if (w == DT_FREE || w == v) break;
+      }
+      if (left == 0 || v == DT_FREE) atomicAdd(bad, 1);
+      code[c][t] = (uint8_t)h;
+    }
 }
 
 // r = b − Q (and its FP32 copy when given), partial r·r
@@ -241,30 +388,6 @@ __global__ void __launch_bounds__(256) k_update_x(Vec3 x, CVec3 P, long long n, 
   }
 }
 
-// the block partial sums of a·b into part[block], no fold (another kernel's fold takes them as its second sum)
-__global__ void __launch_bounds__(256) k_dot_part(CVec3 a, CVec3 b, long long n, double *part, const int *ic) {
-  if (ic[IC_DONE]) return;
-  __shared__ double sh[32];
-  double s = 0.0;
-  for (int cc = 0; cc < 3; cc++)
-#pragma unroll 2
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-      s += a.p[cc][t] * b.p[cc][t];
-  const double r = block_sum(s, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = r;
-}
-
-// P = z + βP (first: P = z)
-__global__ void __launch_bounds__(256, 8) k_pdir(Vec3 P, CVec3 z, long long n, const double *sc, int first, const int *ic) {
-  if (ic && ic[IC_DONE]) return;
-  const double beta = first ? 0.0 : sc[SC_BETA];
-  for (int c = 0; c < 3; c++)
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-      const double zv = z.p[c][t];
-      P.p[c][t] = first ? zv : zv + beta * P.p[c][t];
-    }
-}
-
 // x ← 2x − xprev, xprev ← x (pcg_fast's extrapolated guess, implicit.jl:394-398)
 __global__ void __launch_bounds__(256, 8) k_extrap(Vec3 x, Vec3 xp, long long n) {
   for (int c = 0; c < 3; c++)   // per component (no 64-bit division of the flat index)
@@ -324,6 +447,9 @@ Vec3 vv(double *const *p) {
   return v;
 }
 
+// z is FP32 with the FP32 preconditioner of the fast PCG
+bool zfloat(Ctx *ctx) { return ctx->P.pcg_f32 != 0; }
+
 Fold fold(Ctx *ctx, int mode, int flexible = 0) {
   Fold F;
   F.mode = mode;
@@ -334,10 +460,23 @@ Fold fold(Ctx *ctx, int mode, int flexible = 0) {
   return F;
 }
 // a·b (and a·c) folded into the scalars of `mode`
-void dot2(Ctx *ctx, double *const *a, double *const *b, double *const *c, bool gated, int mode, int flexible = 0) {
+template <class T>
+ZVec3<T> zv(const void *const *p) {
+  ZVec3<T> v;
+  for (int c = 0; c < 3; c++) v.p[c] = p ? (const T *)p[c] : nullptr;
+  return v;
+}
+template <class T>
+void dot2(Ctx *ctx, double *const *a, const void *const *b, const void *const *c, bool gated, int mode, int flexible = 0) {
   PcgDev *S = ctx->pcg;
-  TDGL_LAUNCH(ctx, K_PCG_DOT, (c ? 24.0 : 16.0) * 3 * S->n, k_dot2, S->sblocks, BS, 0, cv(a), cv(b), cv(c ? c : b), c ? 1 : 0, S->n,
-              S->part, gated ? S->ic : nullptr, fold(ctx, mode, flexible));
+  TDGL_LAUNCH(ctx, K_PCG_DOT, (8.0 + (c ? 2 : 1) * sizeof(T)) * 3 * S->n, k_dot2<T>, S->sblocks, BS, 0, cv(a), zv<T>(b),
+              zv<T>(c ? c : b), c ? 1 : 0, S->n, S->part, gated ? S->ic : nullptr, fold(ctx, mode, flexible));
+}
+// r·z (and r·z_old) in z's precision
+void dot_z(Ctx *ctx, const void *const *z, const void *const *zold, int mode, int flexible, bool gated) {
+  PcgDev *S = ctx->pcg;
+  if (zfloat(ctx)) dot2<float>(ctx, S->r, z, zold, gated, mode, flexible);
+  else dot2<double>(ctx, S->r, z, zold, gated, mode, flexible);
 }
 void read_back(Ctx *ctx) {
   PcgDev *S = ctx->pcg;
@@ -346,31 +485,37 @@ void read_back(Ctx *ctx) {
   cudaStreamSynchronize(ctx->stream);
 }
 
-void apply_A(Ctx *ctx, bool gated, int mode) {
+// Q = A P, folded into the scalars of `mode`; with z also P = z + βP from the buffer pold into pnew first
+void apply_A(Ctx *ctx, double *const *P, const void *const *z, double *const *pnew, bool gated, int mode) {
   PcgDev *S = ctx->pcg;
   const Geo &g = ctx->g;
   const tdgl_params &Pp = ctx->P;
   ApplyArgs A;
+  memset(&A, 0, sizeof(A));
   for (int c = 0; c < 3; c++) {
-    A.P[c] = S->P[c];
+    A.P[c] = P[c];
+    A.Z[c] = z ? z[c] : nullptr;
+    A.Pn[c] = pnew ? pnew[c] : nullptr;
     A.D[c] = S->Dp[c];
+    A.Dc[c] = S->Dc[c];
     A.Q[c] = S->Q[c];
   }
+  A.Dt = S->Dt;
   A.sxy = Pp.sxy; A.sxz = Pp.sxz; A.syx = Pp.syx; A.syz = Pp.syz; A.szx = Pp.szx; A.szy = Pp.szy;
-  A.dx = g.dx; A.dy = g.dy; A.dz = g.dz;
   A.iyz = 1.0 / (g.dy * g.dz); A.izx = 1.0 / (g.dz * g.dx); A.ixy = 1.0 / (g.dx * g.dy);
   A.Nx = g.Nx; A.Ny = g.Ny; A.Nz = g.Nz; A.n2 = g.Ny + 1; A.n3 = g.Nz + 1;
+  A.tj = S->tj; A.tk = S->tk; A.ntj = S->ntj; A.ntk = S->ntk; A.chunk = S->chunk;
+  A.sc = S->sc;
   A.part = S->part;
-  A.ic = gated ? S->ic : nullptr;
+  A.ic = S->ic;
+  A.gated = gated;
   A.F = fold(ctx, mode);
-  const double nbox = (double)(g.Nx - 1) * (g.Ny - 1) * (g.Nz - 1);
-  TDGL_LAUNCH(ctx, K_PCG_Q, 72.0 * nbox, k_apply, S->ablocks, BS, 0, A);
-}
-
-void pdir(Ctx *ctx, double *const *z, int first, bool gated) {
-  PcgDev *S = ctx->pcg;
-  TDGL_LAUNCH(ctx, K_PCG_DIR, (first ? 16.0 : 24.0) * 3 * S->n, k_pdir, S->sblocks, BS, 0, vv(S->P), cv(z), S->n, S->sc,
-              first, gated ? S->ic : nullptr);
+  const double nbox = (double)(g.Nx - 1) * (g.Ny - 1) * (g.Nz - 1), zb = zfloat(ctx) ? 4 : 8;
+  const double bytes = 3 * nbox * (8 + 8 + (S->Dc[0] ? 1 : 8) + (z ? 8 + zb : 0));
+  const int grid = S->ntj * S->ntk * S->nchunk;
+  if (!z) TDGL_LAUNCH(ctx, K_PCG_Q, bytes, (k_apply<float, false>), grid, AP_T, apply_smem(S->tj, S->tk), A);
+  else if (zfloat(ctx)) TDGL_LAUNCH(ctx, K_PCG_Q, bytes, (k_apply<float, true>), grid, AP_T, apply_smem(S->tj, S->tk), A);
+  else TDGL_LAUNCH(ctx, K_PCG_Q, bytes, (k_apply<double, true>), grid, AP_T, apply_smem(S->tj, S->tk), A);
 }
 
 int copy3(Ctx *ctx, double *const *dst, double *const *src) {
@@ -391,20 +536,35 @@ int pcg_create(Ctx *ctx) {
   // their partial sums would dominate its microsecond kernels and crowd out concurrent contexts
   const long long per = (long long)BS * 4;
   S->sblocks = (int)std::min<long long>(STR_BLOCKS, std::max<long long>(1, (3 * S->n + per - 1) / per));
-  const long long nbox = (long long)(g.Nx - 1) * (g.Ny - 1) * (g.Nz - 1);
-  S->ablocks = (int)std::min<long long>(RED_BLOCKS, std::max<long long>(1, (nbox + per - 1) / per));
   int rc;
-  double **vecs[9] = {S->P, S->Q, S->x, S->r, S->z, S->b, S->xprev, S->zold, S->Dp};
-  for (int q = 0; q < 9; q++)
+  double **vecs[8] = {S->P[0], S->P[1], S->Q, S->x, S->r, S->b, S->xprev, S->Dp};
+  for (int q = 0; q < 8; q++)
     for (int c = 0; c < 3; c++)
       if ((rc = dalloc(ctx, &vecs[q][c], S->n))) return rc;
-  if ((rc = dalloc(ctx, &S->part, 2 * STR_BLOCKS))) return rc;
+  const size_t zn = ((size_t)S->n * (zfloat(ctx) ? 4 : 8) + 7) / 8;
+  for (int q = 0; q < 2; q++)
+    for (int c = 0; c < 3; c++)
+      if ((rc = dalloc(ctx, (double **)&S->z[q][c], zn))) return rc;
   int dev = 0, nsm = 148;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     nsm = 148;
+  // A·p: tiles of at most AP_TJ rows and AP_T columns, split evenly; as many planes per block as leave one wave of two
+  // blocks per SM (a block also reads the plane before and after its own)
+  const int nj = g.Ny - 1, nk = g.Nz - 1, ni = g.Nx - 1;
+  S->ntj = (nj + AP_TJ - 1) / AP_TJ;
+  S->tj = (nj + S->ntj - 1) / S->ntj;
+  const int tkm = std::max(1, std::min(AP_SUM - S->tj, AP_T / S->tj));
+  S->ntk = (nk + tkm - 1) / tkm;
+  S->tk = (nk + S->ntk - 1) / S->ntk;
+  const int tiles = S->ntj * S->ntk, cols = std::max(1, 2 * nsm / tiles);
+  S->chunk = std::max(1, (ni + cols - 1) / cols);
+  S->nchunk = (ni + S->chunk - 1) / S->chunk;
+  smem_optin(k_apply<float, false>);
+  smem_optin(k_apply<float, true>);
+  smem_optin(k_apply<double, true>);
+  if ((rc = dalloc(ctx, &S->part, 2 * (size_t)std::max(STR_BLOCKS, tiles * S->nchunk)))) return rc;
   // two blocks per SM at most: they fit beside a preconditioner transform block on every SM
   S->xblocks = std::min(S->sblocks, 2 * nsm);
-  if ((rc = dalloc(ctx, &S->part2, S->xblocks))) return rc;
   TDGL_CUDA(cudaStreamCreateWithFlags(&S->side, cudaStreamNonBlocking));
   TDGL_CUDA(cudaEventCreateWithFlags(&S->ev_fork, cudaEventDisableTiming));
   TDGL_CUDA(cudaEventCreateWithFlags(&S->ev_join, cudaEventDisableTiming));
@@ -417,7 +577,18 @@ int pcg_create(Ctx *ctx) {
   // σ_l/σ_n on the ranges, plane-major, for A·p
   const double *D[3] = {ctx->D[0], ctx->D[1], ctx->D[2]};
   to_planes(ctx, D, nullptr, S->Dp);
+  // as byte codes where they have at most 256 values
+  for (int c = 0; c < 3; c++)
+    if ((rc = dalloc(ctx, &S->Dc[c], S->n))) return rc;
+  if ((rc = dalloc(ctx, &S->Dt, 256))) return rc;
+  CVec3 dv = cv(S->Dp);
+  k_dtab_clear<<<1, 256, 0, ctx->stream>>>((unsigned long long *)S->Dt, S->ic);
+  k_dtab<<<S->sblocks, BS, 0, ctx->stream>>>(dv, S->n, (unsigned long long *)S->Dt, S->Dc[0], S->Dc[1], S->Dc[2], S->ic);
+  int bad = 0;
+  TDGL_CUDA(cudaMemcpyAsync(&bad, S->ic, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   TDGL_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (bad)
+    for (int c = 0; c < 3; c++) S->Dc[c] = nullptr;
   return 0;
 }
 
@@ -489,23 +660,30 @@ bool pcg_steady(Ctx *ctx) {
   return S->warm && (!ext || S->have2);
 }
 
-// One PCG iteration (implicit.jl:416-437 with the flexible β of :299-305): q = Ap, α; x, r; z = M⁻¹r; β; p.  Every
-// kernel returns at once after the convergence flag is set.
-static void iteration(Ctx *ctx, double *zc[3], double *zp[3], bool flex, F3 r32, bool r32_ready, double wb32) {
+// The buffers of an iteration: z and the z before, p and the p before; each pair alternates.
+struct Bufs {
+  const void *z[2][3];
+  double *p[2][3];
+  void swap(int which) {
+    for (int c = 0; c < 3; c++) {
+      if (which == 0) std::swap(z[0][c], z[1][c]);
+      else std::swap(p[0][c], p[1][c]);
+    }
+  }
+};
+
+// One PCG iteration (implicit.jl:416-437 with the flexible β of :299-305): p = z + βp, q = Ap, α; x, r; z = M⁻¹r; β.
+// Every kernel returns at once after the convergence flag is set.  In: z[0] is M⁻¹r, p[0] the old direction; out the
+// same for the next one.
+static void iteration(Ctx *ctx, Bufs &B, bool flex, F3 r32, bool r32_ready, double wb32) {
   PcgDev *S = ctx->pcg;
-  apply_A(ctx, true, 3);
+  apply_A(ctx, B.p[0], B.z[0], B.p[1], true, 3);
+  B.swap(1);
   TDGL_LAUNCH(ctx, K_PCG_UPD, (24.0 + wb32) * 3 * S->n, k_update, S->sblocks, BS, 0, vv(S->r), cv(S->Q), S->n, S->sc,
               S->part, S->ic, r32, fold(ctx, 5));
-  // with TDGL_PCG_DOTFUSE=1 the FP32 preconditioner's inverse transform folds r·z and r·z_old (β) as it writes z;
-  // otherwise (the default) r·z_old beside the preconditioner and r·z after it
-  static const bool fuse = [] {
-    const char *e = getenv("TDGL_PCG_DOTFUSE");
-    return e && e[0] == '1';
-  }();
-  const bool fused = flex && fuse;
-  // x += αP and r·z_old need nothing the preconditioner computes: they run on a second stream beside its
-  // compute-bound transforms (one parallel branch of a captured loop), joined before β and the new direction.  When
-  // the launches are timed one by one, the same kernels run in the same order on the one stream.
+  // x += αP needs nothing the preconditioner computes: it runs on a second stream beside its compute-bound transforms
+  // (one parallel branch of a captured loop), joined before β.  When the launches are timed one by one, the same
+  // kernels run in the same order on the one stream.
   const bool side = ctx->branches && !ctx->prof.on;
   cudaStream_t main = ctx->stream;
   if (side) {
@@ -513,39 +691,30 @@ static void iteration(Ctx *ctx, double *zc[3], double *zp[3], bool flex, F3 r32,
     cudaStreamWaitEvent(S->side, S->ev_fork, 0);
     ctx->stream = S->side;
   }
-  TDGL_LAUNCH(ctx, K_PCG_XUPD, 24.0 * 3 * S->n, k_update_x, S->xblocks, BS, 0, vv(S->x), cv(S->P), S->n, S->sc, S->ic);
-  if (flex && !fused)
-    TDGL_LAUNCH(ctx, K_PCG_DOTS, 16.0 * 3 * S->n, k_dot_part, S->xblocks, BS, 0, cv(S->r), cv(zp), S->n, S->part2, S->ic);
+  TDGL_LAUNCH(ctx, K_PCG_XUPD, 24.0 * 3 * S->n, k_update_x, S->xblocks, BS, 0, vv(S->x), cv(B.p[0]), S->n, S->sc, S->ic);
   if (side) {
     ctx->stream = main;
     cudaEventRecord(S->ev_join, S->side);
   }
-  DotFuse df;
-  for (int c = 0; c < 3; c++) {
-    df.r[c] = S->r[c];
-    df.zold[c] = flex ? zp[c] : zc[c];
-  }
-  df.part = S->part;
-  df.F = fold(ctx, 4, flex);
-  const bool folded = sep_apply(ctx, S->r, zc, flex, S->ic, r32_ready, fused ? &df : nullptr);
+  B.swap(0);   // the new z takes the older buffer
+  sep_apply(ctx, S->r, (void *const *)B.z[0], zfloat(ctx), S->ic, r32_ready);
   if (side) cudaStreamWaitEvent(main, S->ev_join, 0);
-  if (!folded) {
-    Fold F = fold(ctx, 4, flex);
-    if (flex) {   // the second sum, r·z_old, from k_dot_part's partials
-      F.bpart = S->part2;
-      F.nbb = S->xblocks;
+  dot_z(ctx, B.z[0], flex ? B.z[1] : nullptr, 4, flex, true);
+}
+
+static Bufs bufs(PcgDev *S) {
+  Bufs B;
+  for (int q = 0; q < 2; q++)
+    for (int c = 0; c < 3; c++) {
+      B.z[q][c] = S->z[q][c];
+      B.p[q][c] = S->P[q][c];
     }
-    TDGL_LAUNCH(ctx, K_PCG_DOT, 16.0 * 3 * S->n, k_dot2, S->sblocks, BS, 0, cv(S->r), cv(zc), cv(zc), 0, S->n, S->part,
-                S->ic, F);
-  }
-  pdir(ctx, zc, 0, true);
-  if (flex)
-    for (int c = 0; c < 3; c++) std::swap(zc[c], zp[c]);
+  return B;
 }
 
 // The loop of a captured step: a conditional WHILE node whose body is BATCH iterations and the kernel that updates
 // the condition (the device decides when the solve is done, as the host did between batches).
-static int loop_graph(Ctx *ctx, double *zc[3], double *zp[3], bool flex, F3 r32, bool r32_ready, double wb32) {
+static int loop_graph(Ctx *ctx, Bufs &B, bool flex, F3 r32, bool r32_ready, double wb32) {
   PcgDev *S = ctx->pcg;
   const int maxit = ctx->P.pcg_maxit;
   cudaStreamCaptureStatus cs;
@@ -569,7 +738,7 @@ static int loop_graph(Ctx *ctx, double *zc[3], double *zp[3], bool flex, F3 r32,
   ctx->stream = ctx->cap_stream;
   cudaError_t e = cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    for (int q = 0; q < BATCH; q++) iteration(ctx, zc, zp, flex, r32, r32_ready, wb32);
+    for (int q = 0; q < BATCH; q++) iteration(ctx, B, flex, r32, r32_ready, wb32);
     TDGL_LAUNCH(ctx, K_PCG_FINAL, 0.0, k_loop_turn, 1, 32, 0, h, S->ic, S->stat, BATCH, maxit);
     cudaGraph_t out = nullptr;
     e = cudaStreamEndCapture(ctx->stream, &out);
@@ -588,12 +757,11 @@ static int pcg_settled(Ctx *ctx) {
   int rc;
   to_planes(ctx, ctx->ph, ctx->th, S->b);
   scale_increment(ctx);
-  dot2(ctx, S->b, S->b, nullptr, false, 0);
+  dot2<double>(ctx, S->b, (const void *const *)S->b, nullptr, false, 0);
   TDGL_CUDA(cudaMemsetAsync(S->ic, 0, IC_N * sizeof(int), ctx->stream));
   TDGL_LAUNCH(ctx, K_PCG_EXTRAP, (ext ? 32.0 : 0.0) * 3 * S->n, k_guess, S->sblocks, BS, 0, vv(S->x), vv(S->xprev), S->n,
               S->sc, S->ic, ext ? 1 : 0);
-  if ((rc = copy3(ctx, S->P, S->x))) return rc;
-  apply_A(ctx, false, -1);
+  apply_A(ctx, S->x, nullptr, nullptr, false, -1);
   F3 r32 = {{nullptr, nullptr, nullptr}};
   float *const *r32p = fast && f32 ? sep_r32(ctx) : nullptr;
   if (r32p)
@@ -602,23 +770,16 @@ static int pcg_settled(Ctx *ctx) {
   TDGL_LAUNCH(ctx, K_PCG_RES, (24.0 + wb32) * 3 * S->n, k_residual, S->sblocks, BS, 0, vv(S->r), cv(S->b), cv(S->Q), S->n,
               S->part, r32, fold(ctx, 1));
   const bool flex = fast && f32;
-  double *zc[3], *zp[3];
-  for (int c = 0; c < 3; c++) {
-    zc[c] = S->z[c];
-    zp[c] = S->zold[c];
-  }
-  sep_apply(ctx, S->r, zc, flex, S->ic, r32p != nullptr);
-  pdir(ctx, zc, 1, true);
-  dot2(ctx, S->r, zc, nullptr, true, 2);
-  if (flex)
-    for (int c = 0; c < 3; c++) std::swap(zc[c], zp[c]);
+  Bufs B = bufs(S);
+  sep_apply(ctx, S->r, (void *const *)B.z[0], zfloat(ctx), S->ic, r32p != nullptr);
+  dot_z(ctx, B.z[0], nullptr, 2, 0, true);
   if (ctx->capturing) {
-    if ((rc = loop_graph(ctx, zc, zp, flex, r32, r32p != nullptr, wb32))) return rc;
+    if ((rc = loop_graph(ctx, B, flex, r32, r32p != nullptr, wb32))) return rc;
   } else {
     int launched = 0;
     while (launched < P.pcg_maxit) {
       const int nb_it = std::min(BATCH, P.pcg_maxit - launched);
-      for (int q = 0; q < nb_it; q++) iteration(ctx, zc, zp, flex, r32, r32p != nullptr, wb32);
+      for (int q = 0; q < nb_it; q++) iteration(ctx, B, flex, r32, r32p != nullptr, wb32);
       launched += nb_it;
       read_back(ctx);
       if (S->host_ic[IC_DONE]) break;
@@ -640,7 +801,7 @@ int pcg_implicit(Ctx *ctx) {
   // b = φₑ − θ on the ranges, then φ = θ + (φₑ − θ)/D on every link (implicit.jl:381-388)
   to_planes(ctx, ctx->ph, ctx->th, S->b);
   scale_increment(ctx);
-  dot2(ctx, S->b, S->b, nullptr, false, 0);
+  dot2<double>(ctx, S->b, (const void *const *)S->b, nullptr, false, 0);
   TDGL_CUDA(cudaMemsetAsync(S->ic, 0, IC_N * sizeof(int), ctx->stream));
   read_back(ctx);
   const double nb = std::sqrt(S->host_sc[SC_BB]);
@@ -661,7 +822,7 @@ int pcg_implicit(Ctx *ctx) {
     return 0;
   }
   if (!S->warm) {
-    sep_apply(ctx, S->b, S->x, false, nullptr);
+    sep_apply(ctx, S->b, (void *const *)S->x, false, nullptr);
     S->have2 = false;
   } else if (fast && P.pcg_extrap) {
     if (S->have2) {
@@ -672,8 +833,7 @@ int pcg_implicit(Ctx *ctx) {
     }
   }
   S->warm = true;
-  if ((rc = copy3(ctx, S->P, S->x))) return rc;
-  apply_A(ctx, false, -1);
+  apply_A(ctx, S->x, nullptr, nullptr, false, -1);
   F3 r32 = {{nullptr, nullptr, nullptr}};
   float *const *r32p = fast && f32 ? sep_r32(ctx) : nullptr;
   if (r32p)
@@ -684,22 +844,14 @@ int pcg_implicit(Ctx *ctx) {
   read_back(ctx);
   const double tol = P.pcg_tol * nb;
   if (std::sqrt(S->host_sc[SC_RR]) > tol) {
-    // z alternates between two buffers, so the flexible β's previous z (implicit.jl:299-305) is the other one
     const bool flex = fast && f32;
-    double *zc[3], *zp[3];
-    for (int c = 0; c < 3; c++) {
-      zc[c] = S->z[c];
-      zp[c] = S->zold[c];
-    }
-    sep_apply(ctx, S->r, zc, flex, nullptr, r32p != nullptr);
-    pdir(ctx, zc, 1, false);
-    dot2(ctx, S->r, zc, nullptr, false, 2);
-    if (flex)
-      for (int c = 0; c < 3; c++) std::swap(zc[c], zp[c]);
+    Bufs B = bufs(S);
+    sep_apply(ctx, S->r, (void *const *)B.z[0], zfloat(ctx), nullptr, r32p != nullptr);
+    dot_z(ctx, B.z[0], nullptr, 2, 0, false);
     int launched = 0;
     while (launched < P.pcg_maxit) {
       const int nb_it = std::min(BATCH, P.pcg_maxit - launched);
-      for (int q = 0; q < nb_it; q++) iteration(ctx, zc, zp, flex, r32, r32p != nullptr, wb32);
+      for (int q = 0; q < nb_it; q++) iteration(ctx, B, flex, r32, r32p != nullptr, wb32);
       launched += nb_it;
       read_back(ctx);
       if (S->host_ic[IC_DONE]) break;

@@ -1,6 +1,4 @@
-// pcg.cuh — the device scalars of the PCG field solve and its deterministic reductions, shared by the PCG kernels
-// (pcg.cu) and by the preconditioner's inverse transform (sep.cu), which folds the PCG's r·z and r·z_old into its
-// epilogue.
+// pcg.cuh — the device scalars of the PCG field solve and its deterministic reductions (pcg.cu).
 #pragma once
 
 #include "common.cuh"
@@ -65,8 +63,6 @@ struct Fold {
   double tol = 0.0;
   double *sc = nullptr;
   int *ic = nullptr;
-  const double *bpart = nullptr;   // the second sum's partials from another kernel (nbb of them), if not null
-  int nbb = 0;
 };
 __device__ void fold_last(const Fold &F, const double *part, double *sh) {
   if (F.mode < 0) return;
@@ -81,10 +77,7 @@ __device__ void fold_last(const Fold &F, const double *part, double *sh) {
   const int nb = gridDim.x;
   double a = 0.0, b = 0.0;
   for (int q = threadIdx.x; q < nb; q += blockDim.x) a += __ldcg(part + q);
-  if (F.bpart)
-    for (int q = threadIdx.x; q < F.nbb; q += blockDim.x) b += __ldcg(F.bpart + q);
-  else
-    for (int q = threadIdx.x; q < nb; q += blockDim.x) b += __ldcg(part + nb + q);
+  for (int q = threadIdx.x; q < nb; q += blockDim.x) b += __ldcg(part + nb + q);
   a = block_sum(a, sh);
   __syncthreads();
   b = block_sum(b, sh);
@@ -95,14 +88,5 @@ __device__ void fold_last(const Fold &F, const double *part, double *sh) {
 }
 
 }  // namespace
-
-// r·z and r·z_old of the PCG folded into the preconditioner's inverse transform (which writes z): the transform reads
-// r and z_old where it writes z and reduces the two sums as k_dot2 does (mode 4: β and rz).
-struct DotFuse {
-  const double *r[3] = {nullptr, nullptr, nullptr};
-  const double *zold[3] = {nullptr, nullptr, nullptr};
-  double *part = nullptr;
-  Fold F;
-};
 
 }  // namespace tdgl

@@ -19,7 +19,6 @@
 #include "common.cuh"
 #include "sep.cuh"
 #include "merge.cuh"
-#include "pcg.cuh"
 
 namespace tdgl {
 
@@ -379,7 +378,6 @@ size_t half_smem(int n1, int n2) {
 }
 bool half_fits(int n1, int n2) {
   const HalfGeo G(n1, n2);
-  // 256 bytes of static shared memory (the folded dot products' block reduction) come on top of the dynamic
   return n1 >= 1 && n2 >= 1 && n2 <= 48 && G.C0 + G.C1 <= 48 && half_smem(n1, n2) + 256 <= 227 * 1024;
 }
 
@@ -397,12 +395,13 @@ __device__ __forceinline__ void cp_async16(void *smem, const float *g) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// FWD: points → modes (TOut = float); otherwise modes → points (TOut = double).  Inputs are FP32.  The three
+// FWD: points → modes; otherwise modes → points.  FP32 in and out.  The three
 // components go in one launch: planes are taken in pairs within a component, and a block's consecutive pairs may
 // belong to different components (the block then loads the next component's half blocks); the shared layout is that
 // of the largest geometry, so a plane of the next component can be staged while the current one is computed.
-template <class TOut, bool FWD>
+template <bool FWD>
 __global__ void __launch_bounds__(HX_THREADS, 1) k_half32(HalfMulti M) {
+  typedef float TOut;
   if (M.done && *M.done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   int n1m = 1, n2m = 1, npairs = 0;
@@ -438,7 +437,6 @@ __global__ void __launch_bounds__(HX_THREADS, 1) k_half32(HalfMulti M) {
       for (int j = lane; j < A.n1; j += 32) cp_async(Stg + k * A.n1 + j, in + j + (long long)A.in_ld * k);
   };
   int loaded = -1;
-  double dz = 0.0, dzo = 0.0;   // r·z and r·z_old over this thread's written points (inverse with M.dot)
   for (int v = blockIdx.x; v < npairs; v += gridDim.x) {
     int ci;
     const int u = locate(v, ci);
@@ -587,17 +585,7 @@ __global__ void __launch_bounds__(HX_THREADS, 1) k_half32(HalfMulti M) {
           }
         }
     } else {
-      const long long obase = out - (TOut *)A.out;   // r and z_old have z's layout
-      const double *rr = M.dot ? M.df.r[ci] + obase : nullptr, *zo = M.dot ? M.df.zold[ci] + obase : nullptr;
-      auto put = [&](long long at, float val) {
-        const TOut zv = (TOut)val;
-        out[at] = zv;
-        if (M.dot) {
-          const double rv = rr[at];
-          dz += rv * (double)zv;
-          dzo += rv * zo[at];
-        }
-      };
+      auto put = [&](long long at, float val) { out[at] = val; };
       for (int t = ht; t < nq; t += HX_HALF) {
         const int p = t % G.hS1, qc = t / G.hS1, pp = n1 - 1 - p, qq = n2 - 1 - qc;
         const bool rp = pp != p, cp = qq != qc;   // a partner exists exactly when the odd class has the index
@@ -619,25 +607,17 @@ __global__ void __launch_bounds__(HX_THREADS, 1) k_half32(HalfMulti M) {
     cp_async_wait_all();
     hsync();   // this half's next plane is staged; O2's reads are done before X is rewritten
   }
-  if (!FWD && M.dot) {   // the block's partial sums, folded by the last block (pcg.cuh)
-    __shared__ double sh[32];
-    __syncthreads();
-    const double a = block_sum(dz, sh);
-    __syncthreads();
-    const double b = block_sum(dzo, sh);
-    if (tid == 0) {
-      M.df.part[blockIdx.x] = a;
-      M.df.part[gridDim.x + blockIdx.x] = b;
-    }
-    __syncthreads();
-    fold_last(M.df.F, M.df.part, sh);
-  }
 }
 
 // r32 = (float)r on the ranges' planes (the forward transform's FP32 input, when the caller has none)
 __global__ void k_to_f32(const double *r, float *r32, long long n) {
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
     r32[t] = (float)r[t];
+}
+
+__global__ void k_widen(const float *z, double *out, long long n) {
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
+    out[t] = (double)z[t];
 }
 
 // ---------------------------------------------------------------------------------------------- the line solve
@@ -1150,12 +1130,12 @@ void half_tx(Ctx *ctx, const HalfMulti &M, bool fwd) {
     npairs += (A.nplanes + 1) / 2;
     n1m = std::max(n1m, A.n1);
     n2m = std::max(n2m, A.n2);
-    bytes += (double)A.nplanes * A.n1 * A.n2 * (fwd ? 2 * sizeof(float) : sizeof(float) + sizeof(double));
+    bytes += (double)A.nplanes * A.n1 * A.n2 * 2 * sizeof(float);
   }
   const int grid = npairs < nsm ? npairs : nsm;
   if (grid <= 0) return;
-  if (fwd) TDGL_LAUNCH(ctx, K_TX32, bytes, (k_half32<float, true>), grid, HX_THREADS, half_smem(n1m, n2m), M);
-  else TDGL_LAUNCH(ctx, K_TX32I, bytes, (k_half32<double, false>), grid, HX_THREADS, half_smem(n1m, n2m), M);
+  if (fwd) TDGL_LAUNCH(ctx, K_TX32, bytes, (k_half32<true>), grid, HX_THREADS, half_smem(n1m, n2m), M);
+  else TDGL_LAUNCH(ctx, K_TX32I, bytes, (k_half32<false>), grid, HX_THREADS, half_smem(n1m, n2m), M);
 }
 
 template <class TIn, class TOut, class T>
@@ -1164,11 +1144,11 @@ void set_plane_smem() {
   smem_optin(k_plane<TIn, TOut, T, 4>);
 }
 
-// z = (I + aK)^{-1} r: r and z are the three plane-major node-shaped component arrays (FP64); entries of z outside
+// z = (I + aK)^{-1} r: r (FP64) and z (T) are the three plane-major node-shaped component arrays; entries of z outside
 // the ranges are not written.
 template <class T>
-void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *const *r, double *const *z, const int *done,
-           const float *const *r32 = nullptr, const DotFuse *dot = nullptr) {
+void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *const *r, T *const *z, const int *done,
+           const float *const *r32 = nullptr) {
   const Geo &g = ctx->g;
   const int nx = S->nx, ny = S->ny, nz = S->nz;
   const long long n2 = g.Ny + 1, n3 = g.Nz + 1, ps = n2 * n3, P = S->P;
@@ -1186,7 +1166,7 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
     A.done = done;
   };
   auto inv = [&](int c, const T *hat, int nj, int nk, int j_off, int k_off, const T *M1t, const T *M2t, int njo, int nko,
-                 double *out, int nplanes) {
+                 T *out, int nplanes) {
     PlaneArgs &A = I.c[c];
     A.in = hat; A.in_base = 0; A.in_ps = P; A.in_ld = ny; A.in_j0 = j_off; A.in_k0 = k_off;
     A.nj_in = nj; A.nk_in = nk;
@@ -1201,9 +1181,6 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
       HalfMulti F, I;
       F.ncomp = I.ncomp = 3;
       F.done = I.done = done;
-      F.dot = 0;
-      I.dot = dot != nullptr;
-      if (dot) I.df = *dot;
       const float *W1f[3] = {b[1].HVf, b[1].HUf, b[1].HVf}, *W2f[3] = {b[2].HVf, b[2].HVf, b[2].HUf};
       const float *W1i[3] = {b[1].HVi, b[1].HUi, b[1].HVi}, *W2i[3] = {b[2].HVi, b[2].HVi, b[2].HUi};
       const float *T1f[3] = {b[1].TVf, b[1].TUf, b[1].TVf}, *T2f[3] = {b[2].TVf, b[2].TVf, b[2].TUf};
@@ -1247,7 +1224,7 @@ void solve(Ctx *ctx, SepDev *S, const Basis<T> *b, Work<T> &w, const double *con
   inv(0, w.Xh, ny, nz, 0, 0, b[1].V, b[2].V, ny, nz, z[0], nx - 1);
   inv(1, w.Yh, ny - 1, nz, 1, 0, b[1].U, b[2].V, ny - 1, nz, z[1], nx);
   inv(2, w.Zh, ny, nz - 1, 0, 1, b[1].V, b[2].U, ny, nz - 1, z[2], nx);
-  plane<T, double, T>(ctx, I);
+  plane<T, T, T>(ctx, I);
 }
 
 // the mode-space arrays of one precision; the FP64 factorisation of the line solves is allocated with the FP64 work
@@ -1486,14 +1463,14 @@ int sep_create(Ctx *ctx) {
   // does not lower the limit of a larger one
   set_plane_smem<double, double, double>();
   set_plane_smem<double, float, float>();
-  set_plane_smem<float, double, float>();
+  set_plane_smem<float, float, float>();
   smem_optin(k_plane_tiled<double, double, double>);
   smem_optin(k_plane_tiled<double, float, float>);
-  smem_optin(k_plane_tiled<float, double, float>);
+  smem_optin(k_plane_tiled<float, float, float>);
   smem_optin(k_linesolve_staged<float>);
   smem_optin(k_linesolve_staged<double>);
-  smem_optin(k_half32<float, true>);
-  smem_optin(k_half32<double, false>);
+  smem_optin(k_half32<true>);
+  smem_optin(k_half32<false>);
   half_tc_init();
   if (!g_sm_count) {
     int dev = 0;
@@ -1510,25 +1487,24 @@ void sep_destroy(Ctx *ctx) {
   ctx->sep = nullptr;
 }
 
-// z = (I + aK)^{-1} r on plane-major component arrays (z may alias r: r is read by the forward pass only)
-bool sep_apply(Ctx *ctx, const double *const *r, double *const *z, bool f32, const int *done, bool r32_ready,
-               const DotFuse *dot) {
+// z = (I + aK)^{-1} r on plane-major component arrays; z in FP32 with f32, else in FP64 (it may then alias r: r is
+// read by the forward pass only)
+void sep_apply(Ctx *ctx, const double *const *r, void *const *z, bool f32, const int *done, bool r32_ready) {
   SepDev *S = ctx->sep;
   if (!f32) {
-    solve<double>(ctx, S, S->bd, S->wd, r, z, done);
-    return false;
+    solve<double>(ctx, S, S->bd, S->wd, r, (double *const *)z, done);
+    return;
   }
-  if (S->r32[0]) {
-    if (!r32_ready) {
-      const long long n = ctx->g.d.n();
-      for (int c = 0; c < 3; c++)
-        TDGL_LAUNCH(ctx, K_CONVERT, 12.0 * n, k_to_f32, nblk(n, BS), BS, 0, r[c], S->r32[c], n);
-    }
-    solve<float>(ctx, S, S->bf, S->wf, r, z, done, S->r32, dot);
-    return dot != nullptr;
+  if (S->r32[0] && !r32_ready) {
+    const long long n = ctx->g.d.n();
+    for (int c = 0; c < 3; c++)
+      TDGL_LAUNCH(ctx, K_CONVERT, 12.0 * n, k_to_f32, nblk(n, BS), BS, 0, r[c], S->r32[c], n);
   }
-  solve<float>(ctx, S, S->bf, S->wf, r, z, done);
-  return false;
+  solve<float>(ctx, S, S->bf, S->wf, r, (float *const *)z, done, S->r32[0] ? S->r32 : nullptr);
+}
+
+void sep_widen(Ctx *ctx, const float *z, double *out, long long n) {
+  TDGL_LAUNCH(ctx, K_CONVERT, 12.0 * n, k_widen, nblk(n, BS), BS, 0, z, out, n);
 }
 
 float *const *sep_r32(Ctx *ctx) { return ctx->sep && ctx->sep->r32[0] ? ctx->sep->r32 : nullptr; }
@@ -1537,7 +1513,7 @@ float *const *sep_r32(Ctx *ctx) { return ctx->sep && ctx->sep->r32[0] ? ctx->sep
 void sep_implicit(Ctx *ctx) {
   SepDev *S = ctx->sep;
   to_planes(ctx, ctx->ph, ctx->th, S->B);
-  sep_apply(ctx, S->B, S->B, false, nullptr);
+  sep_apply(ctx, S->B, (void *const *)S->B, false, nullptr);
   from_planes(ctx, S->B, ctx->th, ctx->ph);
 }
 

@@ -2,7 +2,6 @@
 // the host side; sep_tc.cu: the tensor-core kernel).
 #pragma once
 #include "common.cuh"
-#include "pcg.cuh"
 
 #include <vector>
 
@@ -50,8 +49,6 @@ struct HalfMulti {
   HalfArgs c[3];
   int ncomp;
   const int *done;             // skip when the PCG has converged (null: always run)
-  int dot;                     // inverse only: fold r·z and r·z_old (DotFuse) over the written points
-  DotFuse df;
 };
 
 // The same transforms for planes too large for one block (sep_half.cu): a direction of the three components through X /

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) k_unpair(const __grid_constant__ PairArgs
   if (e >= G.hS1 * G.hS2) return;
   const int qc = e / G.hS1, p = e - qc * G.hS1, pp = n1 - 1 - p, qq = n2 - 1 - qc;
   const float *o2 = P.X[blockIdx.z] + q * P.xps;
-  double *out = (double *)A.out + A.out_base + q * A.out_ps + A.out_j0 + (long long)A.out_ld * A.out_k0;
+  float *out = (float *)A.out + A.out_base + q * A.out_ps + A.out_j0 + (long long)A.out_ld * A.out_k0;
   const bool rp = pp != p, cp = qq != qc;
   const float ee = o2[p + (long long)JP * qc];
   const float eo = cp ? o2[p + (long long)JP * (G.C0 + qc)] : 0.f;
@@ -232,11 +232,11 @@ __global__ void __launch_bounds__(256) k_unpair(const __grid_constant__ PairArgs
   const float oo = rp && cp ? o2[G.R0 + p + (long long)JP * (G.C0 + qc)] : 0.f;
   const float s0 = ee + oe, s1 = eo + oo, d0 = ee - oe, d1 = eo - oo;
   const long long oq = (long long)A.out_ld * qc, oqq = (long long)A.out_ld * qq;
-  out[oq + p] = (double)(s0 + s1);
-  if (rp) out[oq + pp] = (double)(d0 + d1);
+  out[oq + p] = s0 + s1;
+  if (rp) out[oq + pp] = d0 + d1;
   if (cp) {
-    out[oqq + p] = (double)(s0 - s1);
-    if (rp) out[oqq + pp] = (double)(d0 - d1);
+    out[oqq + p] = s0 - s1;
+    if (rp) out[oqq + pp] = d0 - d1;
   }
 }
 
@@ -318,7 +318,7 @@ void half_large(Ctx *ctx, const HalfMulti &M, bool fwd, const double *const *in6
   } else {
     launch<ROW_I>(ctx, R, cat, 8.0 * pts);
     launch<COL_I>(ctx, C, cat, 8.0 * pts);
-    TDGL_LAUNCH(ctx, cat, 12.0 * pts, k_unpair, gp, 256, 0, Q);
+    TDGL_LAUNCH(ctx, cat, 8.0 * pts, k_unpair, gp, 256, 0, Q);
   }
 }
 

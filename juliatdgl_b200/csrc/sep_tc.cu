@@ -111,7 +111,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_half_tc(HalfMulti M, TcSplit 
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ uint32_t tslot;
   __shared__ __align__(8) uint64_t bars[3];
-  __shared__ double shred[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quarter = warp & 3, half = warp >> 2;
   int ci = 0;
   while (ci + 1 < M.ncomp && (int)blockIdx.x >= T.cta0[ci + 1]) ci++;
@@ -119,7 +118,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_half_tc(HalfMulti M, TcSplit 
   const int nb = T.cta0[ci + 1] - T.cta0[ci], bi = (int)blockIdx.x - T.cta0[ci];
   const int q0 = (int)((long long)A.nplanes * bi / nb), q1 = (int)((long long)A.nplanes * (bi + 1) / nb);
   const int cnt = q1 - q0;
-  double dz = 0.0, dzo = 0.0;   // r·z and r·z_old over this thread's written points (inverse with M.dot)
   if (cnt > 0) {
     const TcLayout L(A.n1, A.n2);
     const int n1 = A.n1, n2 = A.n2;
@@ -342,17 +340,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_half_tc(HalfMulti M, TcSplit 
             }
           }
       } else {     // points: the four class entries of (p, qc) unpaired into the mirror quadrant
-        const long long obase = out - (TOut *)A.out;   // r and z_old have z's layout
-        const double *rr = M.dot ? M.df.r[ci] + obase : nullptr, *zo = M.dot ? M.df.zold[ci] + obase : nullptr;
-        auto put = [&](long long at, float val) {
-          const TOut zv = (TOut)val;
-          out[at] = zv;
-          if (M.dot) {
-            const double rv = rr[at];
-            dz += rv * (double)zv;
-            dzo += rv * zo[at];
-          }
-        };
+        auto put = [&](long long at, float val) { out[at] = val; };
         const int pp = n1 - 1 - p;
         const bool pin = p < L.hS1, rp = pin && pp != p;
         if (rows)
@@ -400,18 +388,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_half_tc(HalfMulti M, TcSplit 
     __syncthreads();
     if (warp == 0) umma::tmem_free(tm, 512);
   }
-  if (!FWD && M.dot) {   // the block's partial sums, folded by the last block (pcg.cuh)
-    __syncthreads();
-    const double a = block_sum(dz, shred);
-    __syncthreads();
-    const double b = block_sum(dzo, shred);
-    if (tid == 0) {
-      M.df.part[blockIdx.x] = a;
-      M.df.part[gridDim.x + blockIdx.x] = b;
-    }
-    __syncthreads();
-    fold_last(M.df.F, M.df.part, shred);
-  }
 }
 
 size_t tc_smem(int n1, int n2) { return (size_t)TcLayout(n1, n2).end; }
@@ -427,7 +403,7 @@ bool half_tc_fits(int n1, int n2) {
 
 void half_tc_init() {
   smem_optin(k_half_tc<float, true>);
-  smem_optin(k_half_tc<double, false>);
+  smem_optin(k_half_tc<float, false>);
 }
 
 void half_tc(Ctx *ctx, const HalfMulti &M, bool fwd, long long *err) {
@@ -439,7 +415,7 @@ void half_tc(Ctx *ctx, const HalfMulti &M, bool fwd, long long *err) {
     const HalfArgs &A = M.c[c];
     tot += A.nplanes;
     smem = std::max(smem, tc_smem(A.n1, A.n2));
-    bytes += (double)A.nplanes * A.n1 * A.n2 * (fwd ? 2 * sizeof(float) : sizeof(float) + sizeof(double));
+    bytes += (double)A.nplanes * A.n1 * A.n2 * 2 * sizeof(float);
   }
   if (tot <= 0) return;
   // blocks per component in proportion to its planes, at least one each
@@ -454,7 +430,7 @@ void half_tc(Ctx *ctx, const HalfMulti &M, bool fwd, long long *err) {
   }
   T.cta0[3] = at;
   if (fwd) TDGL_LAUNCH(ctx, K_TX32, bytes, (k_half_tc<float, true>), at, TC_THREADS, smem, M, T);
-  else TDGL_LAUNCH(ctx, K_TX32I, bytes, (k_half_tc<double, false>), at, TC_THREADS, smem, M, T);
+  else TDGL_LAUNCH(ctx, K_TX32I, bytes, (k_half_tc<float, false>), at, TC_THREADS, smem, M, T);
 }
 
 }  // namespace tdgl
