@@ -94,6 +94,15 @@ struct BandPtrs {
   const cd *p[TDGL_MAXB];
 };
 
+namespace tdgl {
+// The first statement of a kernel that may be launched early (programmatic dependent launch, see launch_kernel): lets
+// the next kernel's blocks start once all of this one's have, then waits until everything before it has finished.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+}  // namespace tdgl
+
 // The block a thread works on, as its own launch sees it (blockIdx, gridDim): the hardware's in a plain launch, one
 // context's share of the grid in a merged launch (merge.cuh).  Kernel bodies index with it instead of blockIdx.
 struct Blk {
@@ -309,14 +318,44 @@ void tape_record(Ctx *ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t sme
   t->recs.push_back(std::move(r));
 }
 
+// A launch whose blocks may become resident while the kernel before it in the stream drains: every kernel that is
+// launched so begins with pdl_enter(), which waits for that kernel to finish before it touches memory, so the order of
+// the work is that of plain launches.  What it hides is the launch latency between two kernels of the solvers' loops
+// (pcg.cu, qp.cu and the preconditioner's transforms), at most two blocks per SM: 40 steps 63.8 → 61.3 ms (two fluids,
+// 40×20×8 cells), 18.7 → 18.2 (the ramp, 64×32×8), 229.3 → 223.1 (256×128×32).  Larger grids gain nothing, and the
+// kernels outside the loops lose (192×64×16 without padding: 6514 → 6838 µs): blocks that wait early keep the bands'
+// parallel branches off the SMs, and those of a wide kernel gather on the SMs that drain first.
+const long long EARLY_BLOCKS = 296;
+template <class... P, class... A>
+void launch_kernel(Ctx *ctx, bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A &&...a) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = ctx->stream;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = early && !ctx->prof.on && (long long)grid.x * grid.y * grid.z <= EARLY_BLOCKS ? 1 : 0;
+  cudaLaunchKernelEx(&c, kern, static_cast<A &&>(a)...);   // an error surfaces at the call's cudaGetLastError
+}
+#ifdef TDGL_PDL
+#define TDGL_EARLY true
+#else
+#define TDGL_EARLY false
+#endif
+
 // Every kernel launch of the library goes through this macro: it counts the launch and, when profiling is on,
 // times it with a pair of events on the context's stream; a batch capturing the step also records it.
-#define TDGL_LAUNCH(ctx, cat, bytes, kern, grid, block, smem, ...)        \
+#define TDGL_LAUNCH(ctx, cat, bytes, kern, grid, block, smem, ...) \
+  TDGL_LAUNCH_AS(TDGL_EARLY, ctx, cat, bytes, kern, grid, block, smem, __VA_ARGS__)
+#define TDGL_LAUNCH_AS(early, ctx, cat, bytes, kern, grid, block, smem, ...) \
   do {                                                                   \
     if ((ctx)->tape)                                                     \
       tdgl::tape_record((ctx), kern, dim3(grid), dim3(block), (size_t)(smem), __VA_ARGS__); \
     cudaEvent_t ev_a_ = tdgl::prof_begin(ctx);                           \
-    kern<<<(grid), (block), (smem), (ctx)->stream>>>(__VA_ARGS__);       \
+    tdgl::launch_kernel((ctx), (early), kern, dim3(grid), dim3(block), (size_t)(smem), __VA_ARGS__); \
     tdgl::prof_end((ctx), ev_a_, (cat), (double)(bytes));                \
     (ctx)->launches++;                                                   \
   } while (0)

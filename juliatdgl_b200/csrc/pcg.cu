@@ -15,6 +15,7 @@
 #include <climits>
 #include <cmath>
 
+#define TDGL_PDL   // every kernel launched from this file begins with pdl_enter()
 #include "common.cuh"
 #include "pcg.cuh"
 
@@ -69,6 +70,7 @@ struct ZVec3 {
 };
 template <class T>
 __global__ void __launch_bounds__(256, 8) k_dot2(CVec3 a, ZVec3<T> b, ZVec3<T> c, int use_c, long long n, double *part, const int *ic, Fold F) {
+  tdgl::pdl_enter();
   if (ic && ic[IC_DONE]) return;
   __shared__ double sh[32];
   double s1 = 0.0, s2 = 0.0;
@@ -139,6 +141,7 @@ struct ApRaw {
 
 template <class TZ, bool DIR>
 __global__ void __launch_bounds__(AP_T, 2) k_apply(const __grid_constant__ ApplyArgs A) {
+  tdgl::pdl_enter();
   if (A.gated && A.ic[IC_DONE]) return;
   __shared__ double sh[32];
   extern __shared__ __align__(16) double apsm[];
@@ -287,10 +290,12 @@ __global__ void __launch_bounds__(AP_T, 2) k_apply(const __grid_constant__ Apply
 // set of bit patterns (a value takes its hash's slot or a later one).  *bad counts the entries that found no place.
 const unsigned long long DT_FREE = 0xfff8dead0000beefULL;   // no value a conductivity has (a NaN with this payload)
 __global__ void k_dtab_clear(unsigned long long *tab, int *bad) {
+  tdgl::pdl_enter();
   tab[threadIdx.x] = DT_FREE;
   if (threadIdx.x == 0) *bad = 0;
 }
 __global__ void k_dtab(CVec3 D, long long n, unsigned long long *tab, uint8_t *c0, uint8_t *c1, uint8_t *c2, int *bad) {
+  tdgl::pdl_enter();
   uint8_t *code[3] = {c0, c1, c2};
   for (int c = 0; c < 3; c++)
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -309,6 +314,7 @@ __global__ void k_dtab(CVec3 D, long long n, unsigned long long *tab, uint8_t *c
 
 // r = b − Q (and its FP32 copy when given), partial r·r
 __global__ void __launch_bounds__(256, 8) k_residual(Vec3 r, CVec3 b, CVec3 Q, long long n, double *part, F3 r32, Fold F) {
+  tdgl::pdl_enter();
   __shared__ double sh[32];
   double s = 0.0;
   for (int c = 0; c < 3; c++)
@@ -330,6 +336,7 @@ __global__ void __launch_bounds__(256, 8) k_residual(Vec3 r, CVec3 b, CVec3 Q, l
 // r −= αQ (and r's FP32 copy when given), partial r·r; the convergence test folded in (x: k_update_x)
 __global__ void __launch_bounds__(256, 8) k_update(Vec3 r, CVec3 Q, long long n, const double *sc, double *part, const int *ic,
                          F3 r32, Fold F) {
+  tdgl::pdl_enter();
   if (ic[IC_DONE]) return;
   __shared__ double sh[32];
   const double alpha = sc[SC_ALPHA];
@@ -354,6 +361,7 @@ __global__ void __launch_bounds__(256, 8) k_update(Vec3 r, CVec3 Q, long long n,
 // in the iteration whose r update met the tolerance and set IC_DONE.  It may run beside the preconditioner (on
 // another stream): nothing there changes IC_ITERS, α, P or x.  Four entries per thread in flight.
 __global__ void __launch_bounds__(256) k_update_x(Vec3 x, CVec3 P, long long n, const double *sc, int *ic) {
+  tdgl::pdl_enter();
   __shared__ int run, last;
   const int it = ic[IC_ITERS];
   if (threadIdx.x == 0) run = ic[IC_XDONE] != it;
@@ -390,6 +398,7 @@ __global__ void __launch_bounds__(256) k_update_x(Vec3 x, CVec3 P, long long n, 
 
 // x ← 2x − xprev, xprev ← x (pcg_fast's extrapolated guess, implicit.jl:394-398)
 __global__ void __launch_bounds__(256, 8) k_extrap(Vec3 x, Vec3 xp, long long n) {
+  tdgl::pdl_enter();
   for (int c = 0; c < 3; c++)   // per component (no 64-bit division of the flat index)
     for (long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (long long)gridDim.x * blockDim.x) {
       const double v = x.p[c][u];
@@ -402,6 +411,7 @@ __global__ void __launch_bounds__(256, 8) k_extrap(Vec3 x, Vec3 xp, long long n)
 // with ‖b‖ = 0 the solution is x = 0 (the extrapolation keeps xₙ as xₙ₋₁) and the solve is done; otherwise, with
 // the extrapolated guess, x ← 2xₙ − xₙ₋₁ and xₙ₋₁ ← xₙ.
 __global__ void __launch_bounds__(256, 8) k_guess(Vec3 x, Vec3 xp, long long n, const double *sc, int *ic, int extrap) {
+  tdgl::pdl_enter();
   const bool zero = sc[SC_BB] == 0.0;
   if (zero && blockIdx.x == 0 && threadIdx.x == 0) ic[IC_DONE] = 1;
   if (!zero && !extrap) return;
@@ -416,9 +426,11 @@ __global__ void __launch_bounds__(256, 8) k_guess(Vec3 x, Vec3 xp, long long n, 
 
 // the loop's condition in a captured step: go on while the solve is not done and maxit is not reached
 __global__ void k_loop_enter(cudaGraphConditionalHandle h, const int *ic, int maxit) {
+  tdgl::pdl_enter();
   if (threadIdx.x == 0) cudaGraphSetConditional(h, (!ic[IC_DONE] && ic[IC_LAUNCHED] < maxit) ? 1u : 0u);
 }
 __global__ void k_loop_turn(cudaGraphConditionalHandle h, int *ic, long long *stat, int batch, int maxit) {
+  tdgl::pdl_enter();
   if (threadIdx.x == 0) {
     ic[IC_LAUNCHED] += batch;
     stat[ST_TURNS] += 1;
@@ -428,6 +440,7 @@ __global__ void k_loop_turn(cudaGraphConditionalHandle h, int *ic, long long *st
 
 // the statistics of one solve (done: the zero-source update, which has no iterations)
 __global__ void k_finish(const int *ic, long long *stat, int done) {
+  tdgl::pdl_enter();
   if (threadIdx.x == 0) {
     const int it = ic[IC_ITERS];
     stat[ST_TOTAL] += it;

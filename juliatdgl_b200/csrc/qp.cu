@@ -14,6 +14,7 @@
 // them is carried.
 #include <algorithm>
 
+#define TDGL_PDL   // every kernel launched from this file begins with pdl_enter()
 #include "common.cuh"
 
 namespace tdgl {
@@ -92,6 +93,7 @@ __device__ __forceinline__ double conv(const SrcArgs &A, int mu, long long o, lo
 // The modes' sources on the nodes of the block (x1..x2+1, y1..y2+1, z1..z2+1); the rest of the region stays 0.  Two
 // bands: C_π/s_π − C_σ/s_σ.  N fluids: m_k = Σ_µ Pinv[k, µ] (C_µ/s_µ − ΣC), summed over µ in order from 0.
 __global__ void k_qp_source(SrcArgs A) {
+  tdgl::pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= A.r.n()) return;
   int i, j, k;
@@ -133,6 +135,7 @@ struct AxisArgs {
 
 // out[.., a, ..] = Σ_b M[a + n·b] in[.., b, ..] along the axis, b in order
 __global__ void k_qp_axis(AxisArgs A) {
+  tdgl::pdl_enter();
   if (A.done && *A.done) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long tot = (long long)A.n1 * A.n2 * A.n3;
@@ -162,6 +165,7 @@ struct MuArgs {
   Dim d;
 };
 __global__ void k_qp_mu(MuArgs A) {
+  tdgl::pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= (long long)A.n1 * A.nj * A.nk) return;
   const int i = (int)(t % A.n1);
@@ -186,6 +190,7 @@ struct TurnArgs {
   Dim d;
 };
 __global__ void k_qp_turn(TurnArgs A) {
+  tdgl::pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= A.r.n()) return;
   int i, j, k;
@@ -271,6 +276,7 @@ __device__ void cg_fold(double *part, double *sc, int *ic, int mode, double tol,
 // S on the cut unknowns set to 0, r = −S, x = 0; ‖r‖ (weighted)
 __global__ void k_cg_init(double *S, const uint8_t *cond, double *r, double *x, CgDims D, double *part, double *sc,
                           int *ic, double tol, int maxit) {
+  tdgl::pdl_enter();
   __shared__ double sh[32];
   double a = 0.0;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < D.n(); t += (long long)gridDim.x * blockDim.x) {
@@ -292,6 +298,7 @@ __global__ void k_cg_init(double *S, const uint8_t *cond, double *r, double *x, 
 // the weighted dots a·b and (with c) a·c, folded by `mode`
 __global__ void k_cg_dot(const double *a, const double *b, const double *c, CgDims D, double *part, double *sc,
                          int *ic, int mode, double tol, int maxit) {
+  tdgl::pdl_enter();
   if (ic[QI_DONE]) return;
   __shared__ double sh[32];
   double s1 = 0.0, s2 = 0.0;
@@ -313,6 +320,7 @@ __global__ void k_cg_dot(const double *a, const double *b, const double *c, CgDi
 
 // z = cond ? −z : 0 (the separable solve projected on the conducting unknowns, with the sign of A)
 __global__ void k_cg_proj(double *z, const uint8_t *cond, CgDims D, const int *ic) {
+  tdgl::pdl_enter();
   if (ic[QI_DONE]) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < D.n()) z[t] = cond[t] == 1 ? -z[t] : 0.0;
@@ -321,6 +329,7 @@ __global__ void k_cg_proj(double *z, const uint8_t *cond, CgDims D, const int *i
 // y = −(σn∇²_c − λ) x on the unknowns (_qp_apply!, exchange.jl:52-84)
 __global__ void k_cg_apply(double *y, const double *x, const uint8_t *cond, CgDims D, double ax, double ay, double az,
                            double lam, const int *ic) {
+  tdgl::pdl_enter();
   if (ic[QI_DONE]) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= D.n()) return;
@@ -367,6 +376,7 @@ struct VarCoef {
   double d;
 };
 __global__ void k_cg_apply_var(double *y, const double *x, const uint8_t *typ, CgDims D, VarCoef V, const int *ic) {
+  tdgl::pdl_enter();
   if (ic[QI_DONE]) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= D.n()) return;
@@ -403,6 +413,7 @@ __global__ void k_cg_apply_var(double *y, const double *x, const uint8_t *typ, C
 // op 0: dst = src; 1: dst = dst − src; 2: x += αp, r −= αq (dst = x, src = p, r, q); 3: p = z + βp (dst = p, src = z)
 __global__ void k_cg_vec(int op, double *dst, const double *src, double *r, const double *q, CgDims D, const double *sc,
                          const int *ic) {
+  tdgl::pdl_enter();
   if (ic[QI_DONE]) return;
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= D.n()) return;
@@ -419,6 +430,7 @@ __global__ void k_cg_vec(int op, double *dst, const double *src, double *r, cons
 
 // δ on the region's nodes from the solution x (always: x = 0 when the source was 0)
 __global__ void k_cg_out(double *delta, const double *x, CgDims D, int j0, int k0, Dim d) {
+  tdgl::pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= D.n()) return;
   const int i = (int)(t % D.n1);
@@ -428,20 +440,24 @@ __global__ void k_cg_out(double *delta, const double *x, CgDims D, int j0, int k
 }
 
 __global__ void k_cg_copy(double *dst, const double *src, long long n) {
+  tdgl::pdl_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < n) dst[t] = src[t];
 }
 
 __global__ void k_cg_enter(cudaGraphConditionalHandle h, const int *ic, int maxit) {
+  tdgl::pdl_enter();
   if (threadIdx.x == 0) cudaGraphSetConditional(h, (!ic[QI_DONE] && ic[QI_LAUNCHED] < maxit) ? 1u : 0u);
 }
 __global__ void k_cg_turn(cudaGraphConditionalHandle h, int *ic, int batch, int maxit) {
+  tdgl::pdl_enter();
   if (threadIdx.x == 0) {
     ic[QI_LAUNCHED] += batch;
     cudaGraphSetConditional(h, (!ic[QI_DONE] && ic[QI_LAUNCHED] < maxit) ? 1u : 0u);
   }
 }
 __global__ void k_cg_count(const int *ic, long long *iters) {
+  tdgl::pdl_enter();
   if (threadIdx.x == 0) *iters += ic[QI_IT];
 }
 

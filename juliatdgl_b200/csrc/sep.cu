@@ -401,6 +401,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // of the largest geometry, so a plane of the next component can be staged while the current one is computed.
 template <bool FWD>
 __global__ void __launch_bounds__(HX_THREADS, 1) k_half32(HalfMulti M) {
+  tdgl::pdl_enter();
   typedef float TOut;
   if (M.done && *M.done) return;
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -1134,8 +1135,8 @@ void half_tx(Ctx *ctx, const HalfMulti &M, bool fwd) {
   }
   const int grid = npairs < nsm ? npairs : nsm;
   if (grid <= 0) return;
-  if (fwd) TDGL_LAUNCH(ctx, K_TX32, bytes, (k_half32<true>), grid, HX_THREADS, half_smem(n1m, n2m), M);
-  else TDGL_LAUNCH(ctx, K_TX32I, bytes, (k_half32<false>), grid, HX_THREADS, half_smem(n1m, n2m), M);
+  if (fwd) TDGL_LAUNCH_AS(true, ctx, K_TX32, bytes, (k_half32<true>), grid, HX_THREADS, half_smem(n1m, n2m), M);
+  else TDGL_LAUNCH_AS(true, ctx, K_TX32I, bytes, (k_half32<false>), grid, HX_THREADS, half_smem(n1m, n2m), M);
 }
 
 template <class TIn, class TOut, class T>

@@ -8,6 +8,7 @@
 // Per plane: X (n1 × n2, class order, column-major), O1 (JP × n2), O2 (JP × (C0 + C1), in X's buffer).
 #include <algorithm>
 
+#define TDGL_PDL   // every kernel launched from this file begins with pdl_enter()
 #include "common.cuh"
 #include "sep.cuh"
 
@@ -56,6 +57,7 @@ __device__ __forceinline__ void cpa16(float *s, const float *g, bool ok) {
 
 template <int MODE>
 __global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HGroups P) {
+  tdgl::pdl_enter();
   if (P.done && *P.done) return;
   const HGroup &G = P.g[blockIdx.z];
   const int m0 = blockIdx.y * G.bm, n0 = blockIdx.x * HG_N;
@@ -189,6 +191,7 @@ struct PairArgs {
   HalfMulti M;
 };
 __global__ void __launch_bounds__(256) k_pair(const __grid_constant__ PairArgs P) {
+  tdgl::pdl_enter();
   if (P.M.done && *P.M.done) return;
   const HalfArgs &A = P.M.c[blockIdx.z];
   const int q = blockIdx.y;
@@ -215,6 +218,7 @@ __global__ void __launch_bounds__(256) k_pair(const __grid_constant__ PairArgs P
 
 // the class entries of each mirror quadrant → its four points
 __global__ void __launch_bounds__(256) k_unpair(const __grid_constant__ PairArgs P) {
+  tdgl::pdl_enter();
   if (P.M.done && *P.M.done) return;
   const HalfArgs &A = P.M.c[blockIdx.z];
   const int q = blockIdx.y;

@@ -107,6 +107,7 @@ struct TcSplit {
 
 template <class TOut, bool FWD>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_half_tc(HalfMulti M, TcSplit T) {
+  tdgl::pdl_enter();
   if (M.done && *M.done) return;
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ uint32_t tslot;
