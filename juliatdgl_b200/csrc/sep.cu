@@ -11,6 +11,7 @@
 // j + (Ny+1)(k + (Nz+1) i) (0-based), so one x-plane is contiguous.  Mode-space ("hat") arrays are [p + P i] with
 // p = my + ny·mz, P = ny·nz.  FP64 for the SepSolver, FP32 for the PCG preconditioner (pcg_f32).
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 
@@ -1451,7 +1452,8 @@ int sep_create(Ctx *ctx) {
   if (large && (rc = dalloc(ctx, (double **)&S->gtmp, (size_t)S->nx * S->ny * S->nz))) return rc;
   if (large && f32 && !S->tc && !half_fits(S->ny, S->nz)) {
     S->hw = half_work(S->ny, S->nz);
-    for (int c = 0; c < 3; c++)
+    // its kernels index a component's arrays with 32 bits (beyond: the dense transform)
+    for (int c = 0; c < 3 && S->nx * std::max(S->hw.x_ps, S->hw.o_ps) < INT_MAX; c++)
       if ((rc = dalloc(ctx, &S->hw.x[c], (size_t)S->nx * S->hw.x_ps)) || (rc = dalloc(ctx, &S->hw.o[c], (size_t)S->nx * S->hw.o_ps)))
         return rc;
   }

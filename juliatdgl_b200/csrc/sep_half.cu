@@ -22,11 +22,13 @@ namespace {
 //
 // What bounds it: FP32 multiply-adds.  A block takes bm outputs (⌈h / 64⌉ equal tiles, rounded to 8: 48 for h = 144,
 // 40 for 73) of HG_N = 128 points, 8 × 8 outputs a thread, so four 128-bit shared loads (six wavefronts a warp) feed
-// 64 multiply-adds; three stages of 16 k in flight by cp.async (37 KB a block, so that registers, not shared memory,
-// limit the blocks per SM).  Before, each component and class had its own launch of 48 × 96 tiles without
-// prefetching: 36 launches of 25 µs per PCG iteration on 97 planes of 287 × 95 points, two blocks per SM each.
+// 64 multiply-adds; three stages of 16 k in flight by cp.async (40 KB a block, so that registers, not shared memory,
+// limit the blocks per SM).  The loads along k are element by element (class rows start at any column), so their places
+// are constants and their predicates one byte count: 96 µs for the row product of 95 planes of 287 × 95 points instead
+// of 111.  Before, each component and class had its own launch of 48 × 96 tiles without prefetching: 36 launches of
+// 25 µs per PCG iteration there, two blocks per SM each.
 enum HMode { ROW_F, ROW_I, COL_F, COL_I };
-const int HG_N = 128, HG_K = 16, HG_ST = 3, HG_WS = 64, HG_DS = HG_N + 4, HG_MAXT = 128;
+const int HG_N = 128, HG_K = 16, HG_ST = 3, HG_WS = 64, HG_DS = HG_N + 12, HG_MAXT = 128;
 
 struct HGroup {
   const float *W;   // [K][ldw], columns beyond the block zero up to ldw (a multiple of 8)
@@ -38,7 +40,7 @@ struct HGroup {
   // geometry
   int n1, n2, hS1, hD1, hS2, R0, JP;
   int cls;          // the class (0 even, 1 odd)
-  long long d_off, d_q, c_off, c_q;
+  int d_off, d_q, c_off, c_q;   // a component's arrays hold fewer than 2^31 entries (sep_create checks)
   int d_ld, c_ld;
 };
 struct HGroups {
@@ -46,17 +48,18 @@ struct HGroups {
   const int *done;
 };
 
-__device__ __forceinline__ void cpa4(float *s, const float *g, bool ok) {
-  const int n = ok ? 4 : 0;
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g), "r"(n) : "memory");
+// n bytes (4 or 0) from g, the rest zero
+__device__ __forceinline__ void cpa4(unsigned s, const float *g, int n) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(s), "l"(g), "r"(n) : "memory");
 }
 __device__ __forceinline__ void cpa16(float *s, const float *g, bool ok) {
   const int n = ok ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(s)), "l"(g), "r"(n) : "memory");
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HGroups P) {
+// NT: the block's threads (2 bm), a constant so that the loads' places in shared memory are
+template <int MODE, int NT>
+__global__ void __launch_bounds__(NT, NT > 96 ? 4 : 5) k_hgemm(const __grid_constant__ HGroups P) {
   tdgl::pdl_enter();
   if (P.done && *P.done) return;
   const HGroup &G = P.g[blockIdx.z];
@@ -65,20 +68,21 @@ __global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HG
   constexpr bool ROW = MODE == ROW_F || MODE == ROW_I;
   __shared__ __align__(16) float Ws[HG_ST][HG_K][HG_WS];
   __shared__ __align__(16) float Ds[HG_ST][HG_K][HG_DS];
-  __shared__ long long dbase[HG_N], cbase[HG_N];   // where point n's data and results start (−1: nothing there)
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int t = tid; t < HG_N; t += nt) {
-    const int n = n0 + t;
-    long long db = -1, cb = -1;
-    if (n < G.N) {
+  __shared__ int dbase[HG_DS], cbase[HG_N];   // where point n's data and results start (cbase −1: no result)
+  const int tid = threadIdx.x;
+  constexpr int nt = NT;
+  for (int t = tid; t < HG_DS; t += nt) {   // beyond the tile or the points: the first point's data, read for nothing
+    const int n = t < HG_N && n0 + t < G.N ? n0 + t : n0;
+    int db, cb = -1;
+    {
       if (ROW) {   // n = (plane q, column c in class order)
         const int q = n / G.n2, c = n - q * G.n2;
-        if (MODE == ROW_F) db = G.d_off + q * G.d_q + (G.cls ? G.hS1 : 0) + (long long)G.n1 * c;
-        else db = G.d_off + q * G.d_q + G.cls + (long long)G.d_ld * (c < G.hS2 ? 2 * c : 2 * (c - G.hS2) + 1);
-        cb = G.c_off + q * G.c_q + (G.cls ? G.R0 : 0) + (long long)G.JP * c;
+        if (MODE == ROW_F) db = G.d_off + q * G.d_q + (G.cls ? G.hS1 : 0) + G.n1 * c;
+        else db = G.d_off + q * G.d_q + G.cls + G.d_ld * (c < G.hS2 ? 2 * c : 2 * (c - G.hS2) + 1);
+        cb = G.c_off + q * G.c_q + (G.cls ? G.R0 : 0) + G.JP * c;
       } else {     // n = (plane q, row r of O1)
         const int q = n / G.JP, r = n - q * G.JP;
-        db = G.d_off + q * G.d_q + r + (long long)G.JP * (G.cls ? G.hS2 : 0);
+        db = G.d_off + q * G.d_q + r + G.JP * (G.cls ? G.hS2 : 0);
         if (MODE == COL_F) {   // row r is mode 2r (even class) or 2(r − R0) + 1; the padding rows have none
           const bool odd = r >= G.R0;
           const int p = odd ? r - G.R0 : r;
@@ -89,7 +93,7 @@ __global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HG
       }
     }
     dbase[t] = db;
-    cbase[t] = cb;
+    if (t < HG_N) cbase[t] = n0 + t < G.N ? cb : -1;
   }
   __syncthreads();
   const int bm4 = G.bm / 4, nk = (G.K + HG_K - 1) / HG_K;
@@ -100,21 +104,21 @@ __global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HG
       const bool ok = k0 + k < G.K && m0 + m < G.ldw;
       cpa16(&Ws[s][k][m], ok ? G.W + (long long)(k0 + k) * G.ldw + m0 + m : G.W, ok);
     }
-    if (ROW) {   // consecutive lanes along k
+    if (ROW) {   // consecutive lanes along k; NT / 16 points at a time (the last ones beyond the tile, into the padding)
       const int k = tid % HG_K;
-      const bool kok = k0 + k < G.K;
-      const long long ko = MODE == ROW_F ? k0 + k : 2 * (k0 + k);
-      for (int n = tid / HG_K; n < HG_N; n += nt / HG_K) {
-        const long long b = dbase[n];
-        const bool ok = kok && b >= 0;
-        cpa4(&Ds[s][k][n], ok ? G.D + b + ko : G.D, ok);
-      }
+      const float *src = G.D + (k0 + k < G.K ? (MODE == ROW_F ? k0 + k : 2 * (k0 + k)) : 0);
+      const int nb = k0 + k < G.K ? 4 : 0;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(&Ds[s][k][tid / HG_K]);
+      const int *db = dbase + tid / HG_K;
+      constexpr int DN = NT / HG_K, U = (HG_N + DN - 1) / DN;
+      static_assert(U * DN <= HG_DS, "the last points' padding");
+#pragma unroll
+      for (int u = 0; u < U; u++) cpa4(dst + 4 * DN * u, src + db[DN * u], nb);
     } else {     // consecutive lanes along the rows, four at a time (JP and the tiles are multiples of 4)
-      const int n = 4 * (tid % (HG_N / 4));
-      const long long b = dbase[n];
+      const int n = 4 * (tid % (HG_N / 4)), b = dbase[n];
       for (int k = tid / (HG_N / 4); k < HG_K; k += nt / (HG_N / 4)) {
-        const bool ok = k0 + k < G.K && b >= 0;
-        cpa16(&Ds[s][k][n], ok ? G.D + b + (long long)G.JP * (k0 + k) : G.D, ok);
+        const bool ok = k0 + k < G.K;
+        cpa16(&Ds[s][k][n], ok ? G.D + b + G.JP * (k0 + k) : G.D, ok);
       }
     }
   };
@@ -157,7 +161,7 @@ __global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HG
     if (ROW) {
 #pragma unroll
       for (int b = 0; b < 4; b++) {
-        const long long cb = cbase[n + b];
+        const int cb = cbase[n + b];
         if (cb < 0 || m >= G.M) continue;
         float *c = G.C + cb + m;
         *reinterpret_cast<float4 *>(c) = make_float4(acc[0][4 * h + b], acc[1][4 * h + b], acc[2][4 * h + b], acc[3][4 * h + b]);
@@ -170,11 +174,11 @@ __global__ void __launch_bounds__(HG_MAXT, 4) k_hgemm(const __grid_constant__ HG
         if (MODE == COL_F) {
 #pragma unroll
           for (int b = 0; b < 4; b++) {
-            const long long cb = cbase[n + b];
-            if (cb >= 0) G.C[cb + (long long)G.c_ld * (2 * (m + a) + G.cls)] = acc[a][4 * h + b];
+            const int cb = cbase[n + b];
+            if (cb >= 0) G.C[cb + G.c_ld * (2 * (m + a) + G.cls)] = acc[a][4 * h + b];
           }
         } else if (cbase[n] >= 0) {
-          *reinterpret_cast<float4 *>(G.C + cbase[n] + (long long)G.JP * (m + a)) =
+          *reinterpret_cast<float4 *>(G.C + cbase[n] + G.JP * (m + a)) =
               make_float4(acc[a][4 * h], acc[a][4 * h + 1], acc[a][4 * h + 2], acc[a][4 * h + 3]);
         }
       }
@@ -262,7 +266,16 @@ void launch(Ctx *ctx, HGroups &P, KCat cat, double bytes) {
     gy = std::max(gy, (g.M + bm - 1) / bm);
   }
   if (!gx) return;
-  TDGL_LAUNCH(ctx, cat, bytes, k_hgemm<MODE>, dim3(gx, gy, 6), 2 * bm, 0, P);
+  const dim3 grid(gx, gy, 6);
+  switch (bm) {   // 16, 24, ... 64
+    case 16: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 32>), grid, 32, 0, P); break;
+    case 24: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 48>), grid, 48, 0, P); break;
+    case 32: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 64>), grid, 64, 0, P); break;
+    case 40: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 80>), grid, 80, 0, P); break;
+    case 48: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 96>), grid, 96, 0, P); break;
+    case 56: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 112>), grid, 112, 0, P); break;
+    default: TDGL_LAUNCH(ctx, cat, bytes, (k_hgemm<MODE, 128>), grid, 128, 0, P); break;
+  }
 }
 
 }  // namespace
