@@ -1542,24 +1542,62 @@ const int NOALLOC_MAXDEV = 64;
 // threads at once may both look it up and store the same address: atomic, so that this is not a data race)
 std::atomic<double *> g_noalloc_ptr[NOALLOC_MAXDEV] = {};
 
-// the DCT-II / DST-I bases of n nodes, written into the scratch (the same formulas upload_basis evaluates on the host)
-__global__ void k_noalloc_basis(double *V, double *Vt, double *U, double *Ut, double *s, int n) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long nn = (long long)n * n;
-  if (t < nn) {
-    const int i = (int)(t % n), k = (int)(t / n);
-    const double ck = k == 0 ? sqrt(1.0 / n) : sqrt(2.0 / n);
-    const double v = ck * cos(M_PI * k * (i + 0.5) / n);
-    V[i + (long long)n * k] = v;
-    Vt[k + (long long)n * i] = v;
-    if (i == 0) s[k] = 2 * sin(M_PI * k / (2.0 * n));
+// Everything a call needs in the scratch before its solve, in one launch: the bases of y and z (upload_basis's
+// formulas), the empty slots of the hat arrays, which must read zero (Y at my = 1, Z at mz = 1; every call finds the
+// previous call's contents), and the line factorisation of k_linefactor in closed form (a ≥ 0).  The leading minors of
+// M are θ_i = g^{i+1} cosh((i + 3/2)λ)/cosh(λ/2) with sinh(λ/2) = 1/(2√g), so the pivot reciprocals are
+//   inv_i = θ_{i−1}/θ_i = (1 + q^{2i+1})/(1 + q^{2i+3}) / (1/2 + √(g + 1/4))²,  q = e^{−λ}   (i < n − 1)
+// and the last, whose diagonal is 1 + g, (1 + q^{2n−1})/(1 − q^{2n}) / (1/2 + √(g + 1/4)).  The recurrence is a chain of nx divisions per line (15 µs at 192
+// cells, with P/128 blocks); two bases, a memset and the chain were four launches.  A call on 192×64×16 cells went from
+// 97 to 79 µs.
+struct NoallocSetup {
+  double *V[2], *Vt[2], *U[2], *Ut[2], *s[2];
+  int n[2];          // ny, nz
+  double *inv, *Y, *Z;
+  int nx;
+  double a;
+  int closed;        // the factorisation here (else k_linefactor)
+};
+__global__ void __launch_bounds__(256) k_noalloc_setup(NoallocSetup S) {
+  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int ny = S.n[0], nz = S.n[1], nx = S.nx;
+  const long long P = (long long)ny * nz;
+  if (t < nx * P) {
+    if (!S.closed) return;
+    const int i = (int)(t / P), p = (int)(t - i * P), my = p % ny, mz = p / ny;
+    const double k2 = 2 * sin(M_PI * my / (2.0 * ny)), k3 = 2 * sin(M_PI * mz / (2.0 * nz));
+    const double g = S.a / (1.0 + S.a * (k2 * k2 + k3 * k3));
+    const double lam = 2 * asinh(0.5 / sqrt(g)), d = 0.5 + sqrt(g + 0.25);
+    auto piv = [&](int q) { return (1 + exp(-(2 * q + 1) * lam)) / ((1 + exp(-(2 * q + 3) * lam)) * (d * d)); };
+    S.inv[t] = i < nx - 1 ? piv(i) : (1 + exp(-(2 * nx - 1) * lam)) / (-expm1(-2 * nx * lam) * d);
+    return;
   }
-  const long long m = (long long)(n - 1) * (n - 1);
-  if (t < m) {
-    const int e = (int)(t % (n - 1)), k = 1 + (int)(t / (n - 1));
-    const double u = -sqrt(2.0 / n) * sin(M_PI * k * (e + 1.0) / n);
-    U[e + (long long)(n - 1) * (k - 1)] = u;
-    Ut[(k - 1) + (long long)(n - 1) * e] = u;
+  t -= nx * P;
+#pragma unroll
+  for (int x = 0; x < 2; x++) {
+    const int n = S.n[x];
+    const long long nn = (long long)n * n;
+    if (t < nn) {
+      const int i = (int)(t % n), k = (int)(t / n);
+      const double ck = k == 0 ? sqrt(1.0 / n) : sqrt(2.0 / n);
+      const double v = ck * cos(M_PI * k * (i + 0.5) / n);
+      S.V[x][i + (long long)n * k] = v;
+      S.Vt[x][k + (long long)n * i] = v;
+      if (i == 0) S.s[x][k] = 2 * sin(M_PI * k / (2.0 * n));
+      if (t < (long long)(n - 1) * (n - 1)) {
+        const int e = (int)(t % (n - 1)), m = 1 + (int)(t / (n - 1));
+        const double u = -sqrt(2.0 / n) * sin(M_PI * m * (e + 1.0) / n);
+        S.U[x][e + (long long)(n - 1) * (m - 1)] = u;
+        S.Ut[x][(m - 1) + (long long)(n - 1) * e] = u;
+      }
+      return;
+    }
+    t -= nn;
+  }
+  if (t < (long long)nx * nz) {          // Y at my = 1 (index 0)
+    S.Y[(t / nz) * P + (t % nz) * ny] = 0.0;
+  } else if ((t -= (long long)nx * nz) < (long long)nx * ny) {   // Z at mz = 1
+    S.Z[(t / ny) * P + t % ny] = 0.0;
   }
 }
 
@@ -1614,6 +1652,7 @@ extern "C" int tdgl_sep_apply_noalloc(const tdgl_grid *g, double a, const double
   double *q = s0;
   auto take = [&](long long n) { double *r = q; q += n; return r; };
   const int nax[2] = {ny, nz};
+  NoallocSetup N;
   for (int ax = 1; ax <= 2; ax++) {
     const int n = nax[ax - 1];
     Basis<double> &B = S.bd[ax];
@@ -1621,16 +1660,19 @@ extern "C" int tdgl_sep_apply_noalloc(const tdgl_grid *g, double a, const double
     B.V = take((long long)n * n); B.Vt = take((long long)n * n);
     B.U = take((long long)(n - 1) * (n - 1)); B.Ut = take((long long)(n - 1) * (n - 1));
     B.s = take(n);
-    k_noalloc_basis<<<nblk((long long)n * n, BS), BS, 0, ctx.stream>>>(B.V, B.Vt, B.U, B.Ut, B.s, n);
+    N.V[ax - 1] = B.V; N.Vt[ax - 1] = B.Vt; N.U[ax - 1] = B.U; N.Ut[ax - 1] = B.Ut; N.s[ax - 1] = B.s;
+    N.n[ax - 1] = n;
   }
   Work<double> &w = S.wd;
   w.Xh = take((nx - 1) * P); w.Yh = take(nx * P); w.Zh = take(nx * P);
   w.inv = take(nx * P);
-  // every call shares the scratch and finds the previous call's contents: the empty slots of the hat arrays (Y at
-  // my = 1, Z at mz = 1) must read zero, so the hat arrays are cleared
-  e = cudaMemsetAsync(w.Xh, 0, (size_t)(3LL * nx - 1) * P * sizeof(double), ctx.stream);
-  if (e != cudaSuccess) return set_err(nullptr, TDGL_ECUDA, "cudaMemsetAsync", e);
-  factor_lines(&ctx, &S, w);
+  N.inv = w.inv; N.Y = w.Yh; N.Z = w.Zh;
+  N.nx = nx;
+  N.a = a;
+  N.closed = a >= 0;
+  const long long nset = nx * P + (long long)ny * ny + (long long)nz * nz + (long long)nx * (ny + nz);
+  k_noalloc_setup<<<nblk(nset, BS), BS, 0, ctx.stream>>>(N);
+  if (!N.closed) factor_lines(&ctx, &S, w);
   solve<double>(&ctx, &S, S.bd, w, b, z, nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(nullptr, TDGL_ECUDA, "tdgl_sep_apply_noalloc launch", e);

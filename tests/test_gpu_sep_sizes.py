@@ -29,3 +29,24 @@ def test_separable_inverse_sizes(nx, ny, nz, f32):
     finally:
         gs.close()
     assert np.max(np.abs(out - ref)) / np.max(np.abs(ref)) <= (2e-6 if f32 else 1e-13)
+
+
+@pytest.mark.parametrize("a", [0.0, 1e-9, 49.5, 1e4])
+@pytest.mark.parametrize("nx,ny,nz", [(2, 2, 2), (3, 5, 4), (33, 6, 9)])
+def test_noalloc_closed_factorisation(nx, ny, nz, a):
+    """The allocation-free inverse, whose line factorisation is in closed form, against the context's recurrence at the
+    same a; the two solves differ by the rounding of pivots of condition 1 + 4a: 1e-15 (1 + 4a), at least 1e-13."""
+    import dataclasses
+
+    from test_zz_no_alloc import _noalloc
+    gr = T.Grid.make(nx, ny, nz, dx=0.5, buf=1)
+    st = T.Stepper.make(T.two_band(xi_ratio=4.0, κ=2.0), gr, T.box_masks(gr), selffield_bc="slab")
+    st.fc = dataclasses.replace(st.fc, a=a)
+    gs = gpu.GPUStepper(st)
+    try:
+        b = np.random.default_rng(8).standard_normal(sep_unknowns(gr))
+        ref = gs.sep_apply(b)
+        out = _noalloc(st, b)
+    finally:
+        gs.close()
+    assert np.max(np.abs(out - ref)) <= max(1e-13, 1e-15 * (1 + 4 * a)) * np.max(np.abs(ref))
