@@ -1094,13 +1094,16 @@ void plane(Ctx *ctx, PlaneMulti M) {
     // the threads busy (at most PL_PPB; at most 56 KB of shared memory, four blocks per SM), used when a block has
     // several planes (a merged launch gives each context fewer blocks); persistent: a block keeps its basis chunks
     // in shared memory for all its planes (about four blocks per SM a component).  Small planes take 2-row tiles.
+    // A run alone has rows to spare for few SMs: chunks of at most PL_JC rows (192×64×16 cells: 6539 µs a cycle; with
+    // one chunk 6918).  A step that a batch records fills the GPU with its other runs' planes: whole planes of at most
+    // 2 PL_JC rows, whose input and second basis are then loaded once (16 runs: 34.5 → 32.1 ms a cycle; the same bits).
     const bool small = njm <= 2 * PL_JC;
     const int nsm = g_sm_count > 0 ? g_sm_count : 148;
     size_t smem = 0;
     int ngy = 1, gx = 1;
     for (int c = 0; c < 3; c++) {
       PlaneArgs &A = M.c[c];
-      const int ny = (A.nj_out + PL_JC - 1) / PL_JC;
+      const int rows = small && ctx->tape ? 2 * PL_JC : PL_JC, ny = (A.nj_out + rows - 1) / rows;
       A.jc = small ? rup4((A.nj_out + ny - 1) / ny) : PL_JC;
       const int ta = small ? 2 : 4;
       const int tiles = (A.jc / ta) * (std::max(rup4(A.nk_in), rup4(A.nk_out)) / 4);
