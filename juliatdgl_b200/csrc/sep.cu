@@ -743,6 +743,9 @@ __device__ __forceinline__ void linesolve_b(const Blk bk, T * const &Xh, T * con
 // Shared rows hold LS2_LINES lines and one pad entry (LS2_ROW): the sweeps' lanes walk chunks of consecutive rows,
 // and an odd row length spreads them over the banks.
 const int LS2_THREADS = 256, LS2_LINES = 8, LS2_ROW = LS2_LINES + 1;
+// nodes per lane: ⌈nx/32⌉, made odd, so that the rows of consecutive lanes fall on distinct banks; both kernels below
+// take it, so that they combine the same chunks
+__host__ __device__ inline int ls_chunk(int nx) { return ((nx + 31) >> 5) | 1; }
 template <class T>
 size_t ls2_smem(int nx) {
   // x, y, z as T; the factorisation inv; for T = float also the FP64 right-hand sides of Y and Z
@@ -809,7 +812,7 @@ __device__ __forceinline__ void linesolve_staged_b(const Blk bk, T * const &Xh, 
   // maps of its chunk of ⌈nx/32⌉ nodes, a warp scan of the 32 maps gives every chunk its entry value, and the lanes
   // then run their chunks: ~2⌈nx/32⌉ + 5 dependent steps per sweep instead of nx
   {
-    const int lane = tid & 31, warp = tid >> 5, C = (nx + 31) >> 5, i0 = lane * C, i1 = min(nx, i0 + C);
+    const int lane = tid & 31, warp = tid >> 5, C = ls_chunk(nx), i0 = min(nx, lane * C), i1 = min(nx, i0 + C);
     for (int pr = warp; pr < 2 * LB; pr += LS2_THREADS / 32) {
       const int lp = pr % LB;
       double *v = pr < LB ? yd : zd;
@@ -879,6 +882,186 @@ __device__ __forceinline__ void linesolve_staged_b(const Blk bk, T * const &Xh, 
   }
 }
 
+// The same solve with a line per warp and both components of a line together: a lane holds its chunk of CM right-hand sides and pivots in registers from the load to the
+// solution, so each is read from shared memory once, and the two components' recurrences, whose multipliers are the
+// same, run interleaved.  What bounds the staged kernel above is the latency of its chains (FP64 multiply and add
+// without contraction) at two blocks per SM; it took the components one after the other, and keeps FP64 right-hand
+// sides in shared memory.  The same operations in the same order: the same bits.  The ramp on 256×128×32 cells:
+// 39 → 33 µs per solve, 95 points of 287 × 95 lines 61 → 46.  Lines of more than 32 × LS3_MAX points take the staged kernel.
+const int LS3_MAX = 13;
+template <class T>
+size_t ls3_smem(int nx) { return (size_t)nx * LS2_ROW * (3 * sizeof(T) + sizeof(double)); }
+
+template <class T, int CM>
+__device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T * const &Yh, T * const &Zh, const double * const &inv, int const &nx, long long const &P, int const &ny, const double * const &sy, const double * const &sz, double const &a, const int * const &done);
+template <class T, int CM>
+__global__ void __launch_bounds__(LS2_THREADS, CM > 5 ? 2 : 3) k_linesolve_warp(T *Xh, T *Yh, T *Zh, const double *inv, int nx, long long P,
+                                                                int ny, const double *sy, const double *sz, double a, const int *done) {
+  linesolve_warp_b<T, CM>(TDGL_BLK, Xh, Yh, Zh, inv, nx, P, ny, sy, sz, a, done);
+}
+#define TDGL_LS3_MERGE(CM) TDGL_MERGEABLE((k_linesolve_warp<double, CM>), (linesolve_warp_b<double, CM>), LS2_THREADS, (CM > 5 ? 2 : 3), false)
+TDGL_LS3_MERGE(1);
+TDGL_LS3_MERGE(3);
+TDGL_LS3_MERGE(5);
+TDGL_LS3_MERGE(7);
+TDGL_LS3_MERGE(9);
+TDGL_LS3_MERGE(11);
+TDGL_LS3_MERGE(13);
+template <class T, int CM>
+__device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T * const &Yh, T * const &Zh, const double * const &inv, int const &nx, long long const &P, int const &ny, const double * const &sy, const double * const &sz, double const &a, const int * const &done) {
+  if (done && *done) return;
+  constexpr int LB = LS2_LINES, RS = LS2_THREADS / LB, DS = LS2_ROW;
+  static_assert(LB == LS2_THREADS / 32, "a warp per line");
+  extern __shared__ __align__(16) unsigned char smraw[];
+  double *ivs = (double *)smraw;   // [nx][DS]
+  T *xs = (T *)(ivs + (size_t)nx * DS), *ys = xs + (size_t)nx * DS, *zs = ys + (size_t)nx * DS;
+  const int tid = threadIdx.x, l = tid % LB, r0 = tid / LB;
+  const long long p = (long long)bk.x * LB + l;
+  const bool valid = p < P;
+  for (int i = r0; i < nx; i += RS) {   // all loads in flight at once (cp.async), then one wait
+    const long long o = p + P * i;
+    const int s = i * DS + l;
+    if (valid) {
+      if (i < nx - 1) cp_async(xs + s, Xh + o);
+      else xs[s] = T(0);
+      cp_async(ys + s, Yh + o);
+      cp_async(zs + s, Zh + o);
+      cp_async(ivs + s, inv + o);
+    }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  const int lane = tid & 31, lp = tid >> 5;
+  const long long pl = (long long)bk.x * LB + lp;
+  if (pl < P) {
+    const int my = (int)(pl % ny), mz = (int)(pl / ny);
+    const double k2 = sy[my], k3 = sz[mz];
+    const double c0 = 1.0 + a * (k2 * k2 + k3 * k3);
+    const double g = a / c0, fy = a * k2 / c0, fz = a * k3 / c0;
+    const double pyy = (1.0 + a * k2 * k2) / c0, pyz = a * k2 * k3 / c0, pzz = (1.0 + a * k3 * k3) / c0;
+    const int i0 = lane * CM;
+    double vy[CM], vz[CM], iv[CM];
+    // right-hand sides
+    double xp = i0 > 0 && i0 <= nx ? (double)xs[(i0 - 1) * DS + lp] : 0.0;
+#pragma unroll
+    for (int u = 0; u < CM; u++) {
+      const int i = i0 + u, s = i * DS + lp;
+      vy[u] = vz[u] = iv[u] = 0.0;
+      if (i < nx) {
+        const double x = (double)xs[s], dtb = xp - x;
+        const double byp = (double)ys[s] + fy * dtb, bzp = (double)zs[s] + fz * dtb;
+        vy[u] = pyy * byp + pyz * bzp;
+        vz[u] = pyz * byp + pzz * bzp;
+        iv[u] = ivs[s];
+        xp = x;
+      }
+    }
+    // forward: d_i = α_i d_{i−1} + β_i (α_i = g inv_i, β_i = rhs_i inv_i), as affine maps scanned over the lanes
+    double A = 1.0, By = 0.0, Bz = 0.0;
+#pragma unroll
+    for (int u = 0; u < CM; u++)
+      if (i0 + u < nx) {
+        const double al = i0 + u > 0 ? g * iv[u] : 0.0;
+        A = al * A;
+        By = al * By + vy[u] * iv[u];
+        Bz = al * Bz + vz[u] * iv[u];
+      }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double Ap = __shfl_up_sync(0xffffffffu, A, o), yp = __shfl_up_sync(0xffffffffu, By, o), zp = __shfl_up_sync(0xffffffffu, Bz, o);
+      if (lane >= o) {
+        By = A * yp + By;
+        Bz = A * zp + Bz;
+        A = A * Ap;
+      }
+    }
+    double dy = __shfl_up_sync(0xffffffffu, By, 1), dz = __shfl_up_sync(0xffffffffu, Bz, 1);
+    if (lane == 0) dy = dz = 0.0;
+#pragma unroll
+    for (int u = 0; u < CM; u++)
+      if (i0 + u < nx) {
+        const double al = i0 + u > 0 ? g * iv[u] : 0.0;
+        dy = al * dy + vy[u] * iv[u];
+        dz = al * dz + vz[u] * iv[u];
+        vy[u] = dy;
+        vz[u] = dz;
+      }
+    // backward: y_i = −c_i y_{i+1} + d_i (c_i = up·inv_i, 0 on the last node)
+    const double ul = -g;
+    A = 1.0;
+    By = Bz = 0.0;
+#pragma unroll
+    for (int u = CM - 1; u >= 0; u--)
+      if (i0 + u < nx) {
+        const double ga = -((i0 + u < nx - 1 ? ul : 0.0) * iv[u]);
+        A = ga * A;
+        By = ga * By + vy[u];
+        Bz = ga * Bz + vz[u];
+      }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double An = __shfl_down_sync(0xffffffffu, A, o), yn = __shfl_down_sync(0xffffffffu, By, o), zn = __shfl_down_sync(0xffffffffu, Bz, o);
+      if (lane + o < 32) {
+        By = A * yn + By;
+        Bz = A * zn + Bz;
+        A = A * An;
+      }
+    }
+    double y = __shfl_down_sync(0xffffffffu, By, 1), z = __shfl_down_sync(0xffffffffu, Bz, 1);
+    if (lane == 31) y = z = 0.0;
+#pragma unroll
+    for (int u = CM - 1; u >= 0; u--)
+      if (i0 + u < nx) {
+        const double ga = -((i0 + u < nx - 1 ? ul : 0.0) * iv[u]);
+        y = ga * y + vy[u];
+        z = ga * z + vz[u];
+        vy[u] = y;
+        vz[u] = z;
+      }
+    // X from Y and Z at the node and the next one (the chunk's last node: the next lane's first; the shuffles also
+    // order every lane's reads of X above before the writes here)
+    double yn = __shfl_down_sync(0xffffffffu, vy[0], 1), zn = __shfl_down_sync(0xffffffffu, vz[0], 1);
+#pragma unroll
+    for (int u = CM - 1; u >= 0; u--) {
+      const int i = i0 + u, s = i * DS + lp;
+      if (i < nx) {
+        if (i < nx - 1) xs[s] = (T)(((double)xs[s] + a * k2 * (yn - vy[u]) + a * k3 * (zn - vz[u])) / c0);
+        ys[s] = (T)vy[u];
+        zs[s] = (T)vz[u];
+        yn = vy[u];
+        zn = vz[u];
+      }
+    }
+  }
+  __syncthreads();
+  if (!valid) return;
+  for (int i = r0; i < nx; i += RS) {
+    const long long o = p + P * i;
+    const int s = i * DS + l;
+    if (i < nx - 1) Xh[o] = xs[s];
+    Yh[o] = ys[s];
+    Zh[o] = zs[s];
+  }
+}
+
+// the warp-per-line kernel for lines of nx points (null: too long)
+template <class T>
+using LineKernel = void (*)(T *, T *, T *, const double *, int, long long, int, const double *, const double *, double, const int *);
+template <class T>
+LineKernel<T> linesolve_warp_kernel(int nx) {
+  static const LineKernel<T> k[] = {k_linesolve_warp<T, 1>, k_linesolve_warp<T, 3>, k_linesolve_warp<T, 5>, k_linesolve_warp<T, 7>,
+                                    k_linesolve_warp<T, 9>, k_linesolve_warp<T, 11>, k_linesolve_warp<T, 13>};
+  const int cm = ls_chunk(nx);
+  return cm <= LS3_MAX && ls3_smem<T>(nx) <= 227 * 1024 ? k[cm / 2] : nullptr;
+}
+// lets the line solves of nx points use their shared memory
+template <class T>
+cudaError_t linesolve_smem(int nx) {
+  const LineKernel<T> k = linesolve_warp_kernel<T>(nx);
+  const cudaError_t e = k ? smem_optin((const void *)k) : cudaSuccess;
+  return e == cudaSuccess ? smem_optin(k_linesolve_staged<T>) : e;
+}
+
 // the FP64 bases' wave numbers s = 2 sin(πk/2n) of y and z, for both precisions
 template <class T>
 void linesolve(Ctx *ctx, SepDev *S, Work<T> &w, const int *done) {
@@ -886,7 +1069,13 @@ void linesolve(Ctx *ctx, SepDev *S, Work<T> &w, const int *done) {
   const long long P = S->P;
   const KCat cat = sizeof(T) == 8 ? K_MODES64 : K_MODES32;
   const double bytes = (6.0 * sizeof(T) + 8.0) * nx * P;   // X, Y, Z in and out; the factorisation in
-  if (ls2_smem<T>(nx) <= 227 * 1024) {
+  // a step that a batch records takes the staged kernel: its chunks have one form for every length, so runs of different
+  // lengths share a merged launch (the same bits)
+  const auto warp = ctx->tape ? nullptr : linesolve_warp_kernel<T>(nx);
+  if (warp) {
+    TDGL_LAUNCH(ctx, cat, bytes, warp, (int)((P + LS2_LINES - 1) / LS2_LINES), LS2_THREADS, ls3_smem<T>(nx), w.Xh, w.Yh, w.Zh, w.inv, nx,
+                P, S->ny, S->bd[1].s, S->bd[2].s, ctx->P.a_imp, done);
+  } else if (ls2_smem<T>(nx) <= 227 * 1024) {
     TDGL_LAUNCH(ctx, cat, bytes, k_linesolve_staged<T>, (int)((P + LS2_LINES - 1) / LS2_LINES), LS2_THREADS,
                 ls2_smem<T>(nx), w.Xh, w.Yh, w.Zh, w.inv, nx, P, S->ny, S->bd[1].s, S->bd[2].s, ctx->P.a_imp,
                 done);
@@ -1473,8 +1662,8 @@ int sep_create(Ctx *ctx) {
   smem_optin(k_plane_tiled<double, double, double>);
   smem_optin(k_plane_tiled<double, float, float>);
   smem_optin(k_plane_tiled<float, float, float>);
-  smem_optin(k_linesolve_staged<float>);
-  smem_optin(k_linesolve_staged<double>);
+  linesolve_smem<float>(S->nx);
+  linesolve_smem<double>(S->nx);
   smem_optin(k_half32<true>);
   smem_optin(k_half32<false>);
   half_tc_init();
@@ -1639,7 +1828,7 @@ extern "C" int tdgl_sep_apply_noalloc(const tdgl_grid *g, double a, const double
   if (e == cudaSuccess)
     e = smem_optin(k_plane<double, double, double, 4>);
   if (e != cudaSuccess) return set_err(nullptr, TDGL_ECUDA, "cudaFuncSetAttribute", e);
-  e = smem_optin(k_linesolve_staged<double>);
+  e = linesolve_smem<double>(nx);
   if (e != cudaSuccess) return set_err(nullptr, TDGL_ECUDA, "cudaFuncSetAttribute", e);
   double *s0 = g_noalloc_ptr[dev].load();
   // a context on the host stack: the stream and the geometry for the launches, nothing on the device

@@ -1,6 +1,6 @@
 """The separable inverse at the edges of its transforms' tiles: extents where the components' row chunks differ in number
 or kind (48 | 49 and 96 | 97 rows), remainders of the register tiles, the smallest planes, and planes that take the batched products (several planes to a
-tile of points, both parities of each extent); FP64 and FP32, against
+tile of points, both parities of each extent), lines of every chunk length (and too long for one warp); FP64 and FP32, against
 the oracle's dense three-axis transforms at the tolerances of the parity test."""
 import numpy as np
 import pytest
@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("f32", [False, True])
 @pytest.mark.parametrize("nx,ny,nz", [(5, 48, 3), (3, 96, 6), (9, 47, 17), (2, 2, 2), (20, 13, 4), (33, 5, 9),
-                                      (3, 64, 64), (2, 63, 70), (6, 100, 55), (2, 140, 49)])
+                                      (3, 64, 64), (2, 63, 70), (6, 100, 55), (2, 140, 49),
+                                      (31, 3, 2), (63, 2, 3), (95, 4, 2), (97, 3, 3), (416, 2, 2), (430, 3, 2)])
 def test_separable_inverse_sizes(nx, ny, nz, f32):
     gr = T.Grid.make(nx, ny, nz, dx=0.5, buf=1)
     md = T.two_band(xi_ratio=4.0, κ=2.0)
