@@ -743,9 +743,8 @@ __device__ __forceinline__ void linesolve_b(const Blk bk, T * const &Xh, T * con
 // Shared rows hold LS2_LINES lines and one pad entry (LS2_ROW): the sweeps' lanes walk chunks of consecutive rows,
 // and an odd row length spreads them over the banks.
 const int LS2_THREADS = 256, LS2_LINES = 8, LS2_ROW = LS2_LINES + 1;
-// nodes per lane: ⌈nx/32⌉, made odd, so that the rows of consecutive lanes fall on distinct banks; both kernels below
-// take it, so that they combine the same chunks
-__host__ __device__ inline int ls_chunk(int nx) { return ((nx + 31) >> 5) | 1; }
+// nodes per lane; both kernels below take it, so that they combine the same chunks and give the same bits
+__host__ __device__ inline int ls_chunk(int nx) { return (nx + 31) >> 5; }
 template <class T>
 size_t ls2_smem(int nx) {
   // x, y, z as T; the factorisation inv; for T = float also the FP64 right-hand sides of Y and Z
@@ -812,7 +811,7 @@ __device__ __forceinline__ void linesolve_staged_b(const Blk bk, T * const &Xh, 
   // maps of its chunk of ⌈nx/32⌉ nodes, a warp scan of the 32 maps gives every chunk its entry value, and the lanes
   // then run their chunks: ~2⌈nx/32⌉ + 5 dependent steps per sweep instead of nx
   {
-    const int lane = tid & 31, warp = tid >> 5, C = ls_chunk(nx), i0 = min(nx, lane * C), i1 = min(nx, i0 + C);
+    const int lane = tid & 31, warp = tid >> 5, C = ls_chunk(nx), i0 = lane * C, i1 = min(nx, i0 + C);
     for (int pr = warp; pr < 2 * LB; pr += LS2_THREADS / 32) {
       const int lp = pr % LB;
       double *v = pr < LB ? yd : zd;
@@ -889,8 +888,12 @@ __device__ __forceinline__ void linesolve_staged_b(const Blk bk, T * const &Xh, 
 // sides in shared memory.  The same operations in the same order: the same bits.  The ramp on 256×128×32 cells:
 // 39 → 33 µs per solve, 95 points of 287 × 95 lines 61 → 46.  Lines of more than 32 × LS3_MAX points take the staged kernel.
 const int LS3_MAX = 13;
+// the row of node i: LS2_ROW entries a node, and one more per chunk of an even length, so that the rows of consecutive
+// lanes are an odd number of entries apart (distinct banks)
+template <int CM>
+__device__ __forceinline__ int ls3_row(int i) { return i * LS2_ROW + (CM % 2 ? 0 : i / CM); }
 template <class T>
-size_t ls3_smem(int nx) { return (size_t)nx * LS2_ROW * (3 * sizeof(T) + sizeof(double)); }
+size_t ls3_smem(int nx) { return ((size_t)nx * LS2_ROW + 32) * (3 * sizeof(T) + sizeof(double)); }
 
 template <class T, int CM>
 __device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T * const &Yh, T * const &Zh, const double * const &inv, int const &nx, long long const &P, int const &ny, const double * const &sy, const double * const &sz, double const &a, const int * const &done);
@@ -899,28 +902,21 @@ __global__ void __launch_bounds__(LS2_THREADS, CM > 5 ? 2 : 3) k_linesolve_warp(
                                                                 int ny, const double *sy, const double *sz, double a, const int *done) {
   linesolve_warp_b<T, CM>(TDGL_BLK, Xh, Yh, Zh, inv, nx, P, ny, sy, sz, a, done);
 }
-#define TDGL_LS3_MERGE(CM) TDGL_MERGEABLE((k_linesolve_warp<double, CM>), (linesolve_warp_b<double, CM>), LS2_THREADS, (CM > 5 ? 2 : 3), false)
-TDGL_LS3_MERGE(1);
-TDGL_LS3_MERGE(3);
-TDGL_LS3_MERGE(5);
-TDGL_LS3_MERGE(7);
-TDGL_LS3_MERGE(9);
-TDGL_LS3_MERGE(11);
-TDGL_LS3_MERGE(13);
 template <class T, int CM>
 __device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T * const &Yh, T * const &Zh, const double * const &inv, int const &nx, long long const &P, int const &ny, const double * const &sy, const double * const &sz, double const &a, const int * const &done) {
   if (done && *done) return;
-  constexpr int LB = LS2_LINES, RS = LS2_THREADS / LB, DS = LS2_ROW;
+  constexpr int LB = LS2_LINES, RS = LS2_THREADS / LB;
+  const int NS = nx * LS2_ROW + 32;   // entries of an array
   static_assert(LB == LS2_THREADS / 32, "a warp per line");
   extern __shared__ __align__(16) unsigned char smraw[];
-  double *ivs = (double *)smraw;   // [nx][DS]
-  T *xs = (T *)(ivs + (size_t)nx * DS), *ys = xs + (size_t)nx * DS, *zs = ys + (size_t)nx * DS;
+  double *ivs = (double *)smraw;
+  T *xs = (T *)(ivs + NS), *ys = xs + NS, *zs = ys + NS;
   const int tid = threadIdx.x, l = tid % LB, r0 = tid / LB;
   const long long p = (long long)bk.x * LB + l;
   const bool valid = p < P;
   for (int i = r0; i < nx; i += RS) {   // all loads in flight at once (cp.async), then one wait
     const long long o = p + P * i;
-    const int s = i * DS + l;
+    const int s = ls3_row<CM>(i) + l;
     if (valid) {
       if (i < nx - 1) cp_async(xs + s, Xh + o);
       else xs[s] = T(0);
@@ -942,10 +938,10 @@ __device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T 
     const int i0 = lane * CM;
     double vy[CM], vz[CM], iv[CM];
     // right-hand sides
-    double xp = i0 > 0 && i0 <= nx ? (double)xs[(i0 - 1) * DS + lp] : 0.0;
+    double xp = i0 > 0 && i0 <= nx ? (double)xs[ls3_row<CM>(i0 - 1) + lp] : 0.0;
 #pragma unroll
     for (int u = 0; u < CM; u++) {
-      const int i = i0 + u, s = i * DS + lp;
+      const int i = i0 + u, s = ls3_row<CM>(i) + lp;
       vy[u] = vz[u] = iv[u] = 0.0;
       if (i < nx) {
         const double x = (double)xs[s], dtb = xp - x;
@@ -1023,7 +1019,7 @@ __device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T 
     double yn = __shfl_down_sync(0xffffffffu, vy[0], 1), zn = __shfl_down_sync(0xffffffffu, vz[0], 1);
 #pragma unroll
     for (int u = CM - 1; u >= 0; u--) {
-      const int i = i0 + u, s = i * DS + lp;
+      const int i = i0 + u, s = ls3_row<CM>(i) + lp;
       if (i < nx) {
         if (i < nx - 1) xs[s] = (T)(((double)xs[s] + a * k2 * (yn - vy[u]) + a * k3 * (zn - vz[u])) / c0);
         ys[s] = (T)vy[u];
@@ -1037,7 +1033,7 @@ __device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T 
   if (!valid) return;
   for (int i = r0; i < nx; i += RS) {
     const long long o = p + P * i;
-    const int s = i * DS + l;
+    const int s = ls3_row<CM>(i) + l;
     if (i < nx - 1) Xh[o] = xs[s];
     Yh[o] = ys[s];
     Zh[o] = zs[s];
@@ -1049,10 +1045,12 @@ template <class T>
 using LineKernel = void (*)(T *, T *, T *, const double *, int, long long, int, const double *, const double *, double, const int *);
 template <class T>
 LineKernel<T> linesolve_warp_kernel(int nx) {
-  static const LineKernel<T> k[] = {k_linesolve_warp<T, 1>, k_linesolve_warp<T, 3>, k_linesolve_warp<T, 5>, k_linesolve_warp<T, 7>,
-                                    k_linesolve_warp<T, 9>, k_linesolve_warp<T, 11>, k_linesolve_warp<T, 13>};
+  static const LineKernel<T> k[] = {k_linesolve_warp<T, 1>, k_linesolve_warp<T, 2>,  k_linesolve_warp<T, 3>,  k_linesolve_warp<T, 4>,
+                                    k_linesolve_warp<T, 5>, k_linesolve_warp<T, 6>,  k_linesolve_warp<T, 7>,  k_linesolve_warp<T, 8>,
+                                    k_linesolve_warp<T, 9>, k_linesolve_warp<T, 10>, k_linesolve_warp<T, 11>, k_linesolve_warp<T, 12>,
+                                    k_linesolve_warp<T, 13>};
   const int cm = ls_chunk(nx);
-  return cm <= LS3_MAX && ls3_smem<T>(nx) <= 227 * 1024 ? k[cm / 2] : nullptr;
+  return cm <= LS3_MAX && ls3_smem<T>(nx) <= 227 * 1024 ? k[cm - 1] : nullptr;
 }
 // lets the line solves of nx points use their shared memory
 template <class T>
