@@ -162,6 +162,8 @@ static int check_params(const tdgl_params *p, char *why, size_t n) {
   if ((double)(g.Nx + 1) * (g.Ny + 1) * (g.Nz + 1) * 3.0 >= 2147483647.0) return no("grid too large");
   if (!(g.x1 >= 2 && g.x2 + 1 <= g.Nx && g.y1 >= 2 && g.y2 + 1 <= g.Ny && g.z1 >= 2 && g.z2 + 1 <= g.Nz))
     return no("the block must have at least one padding cell on each face");
+  // a block one cell thick has no inner node: its ghosts read ghosts, its band stages have nothing to launch
+  if (g.x2 < g.x1 + 1 || g.y2 < g.y1 + 1 || g.z2 < g.z1 + 1) return no("the block must have at least two cells along each axis");
   for (int mu = 0; mu < p->nbands; mu++) {
     if (p->stages[mu] < 0 || p->stages[mu] > TDGL_MAXSTG) return no("stage count out of range");
     if (p->stages[mu] == 0 && p->nsub[mu] < 1) return no("substeps must be >= 1");

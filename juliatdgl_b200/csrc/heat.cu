@@ -117,8 +117,9 @@ __device__ __forceinline__ double heat_node(const HeatArgs &A, double q, double 
   return tn;
 }
 
-// Every node of the block: a face takes the θ inside (copied x, then y, then z, terms.jl:70-78: each index clamped);
-// an inner node its source and old θ by plane, or, with D_T per material, a copy of the field (faces included) in R.
+// Every node of the block: a face takes the θ inside (copied x, then y, then z, terms.jl:70-78: each index clamped; the
+// parameter check refuses a block without inner nodes); an inner node its source and old θ by plane, or, with D_T per
+// material, a copy of the field (faces included) in R.
 __global__ void __launch_bounds__(HT_BS) k_heat_source(const __grid_constant__ HeatArgs A) {
   const int nx1 = A.x2 + 2 - A.x1, ny1 = A.y2 + 2 - A.y1, nz1 = A.z2 + 2 - A.z1;
   const long long t = (long long)blockIdx.x * HT_BS + threadIdx.x;
@@ -230,8 +231,8 @@ int heat_create(Ctx *ctx, const tdgl_materials *M) {
   // the source (with D_T per material by node, else by plane beside the old θ), and the last two planes' θ where they do
   // not fit shared memory
   const Geo &g = ctx->g;
-  const size_t nc = (size_t)std::max(1, g.y2 - g.y1) * std::max(1, g.z2 - g.z1);
-  const size_t np = (size_t)std::max(1, (g.x2 - g.x1) + (g.y2 - g.y1) + (g.z2 - g.z1) - 2) * nc;
+  const size_t nc = (size_t)(g.y2 - g.y1) * (g.z2 - g.z1);
+  const size_t np = (size_t)((g.x2 - g.x1) + (g.y2 - g.y1) + (g.z2 - g.z1) - 2) * nc;
   if ((rc = dalloc(ctx, &ctx->heat_S, ctx->Th2 ? (size_t)nn : np))) return rc;
   if (!ctx->Th2 && (rc = dalloc(ctx, &ctx->heat_Q, np))) return rc;
   if (!ctx->Th2 && 2 * nc * sizeof(double) > HT_SMEM && (rc = dalloc(ctx, &ctx->heat_prev, 2 * nc))) return rc;
@@ -292,7 +293,6 @@ void heat_step(Ctx *ctx) {
   const long long ni = (long long)(g.x2 - g.x1) * (g.y2 - g.y1) * (g.z2 - g.z1), nc = (long long)(g.y2 - g.y1) * (g.z2 - g.z1);
   const long long nb = (long long)(g.x2 + 2 - g.x1) * (g.y2 + 2 - g.y1) * (g.z2 + 2 - g.z1);
   TDGL_LAUNCH(ctx, K_HEAT, nb * (8.0 * 9 + 32.0 * ctx->N), k_heat_source, nblk(nb, HT_BS), HT_BS, 0, A);
-  if (ni <= 0) return;
   if (A.uni) {
     auto pow2 = [](double v) {
       int e;
