@@ -25,7 +25,7 @@ const size_t HT_SMEM = 200 * 1024;   // shared memory for the last two planes
 
 struct HeatArgs {
   double *T;
-  double *Q, *S;        // by plane: the old θ (then the new one) and the source, [s − s0][column] (one D_T)
+  double *Q, *S;        // by plane: the old θ (then the new one) and the source, [(s − s0) mod nx][column] (one D_T)
   double *prev;         // the last two planes' new θ when they do not fit shared memory (2 × columns)
   BandPtrs G, F;
   const double *th[3], *ph[3], *f;
@@ -139,15 +139,18 @@ __global__ void __launch_bounds__(HT_BS) k_heat_source(const __grid_constant__ H
     return;
   }
   const int ny = A.y2 - A.y1, nz = A.z2 - A.z1;
-  const long long w = (long long)((i - A.x1 - 1) + (j - A.y1 - 1) + (k - A.z1 - 1)) * (ny * nz) + (j - A.y1 - 1) + ny * (k - A.z1 - 1);
+  const long long w = (long long)(((i - A.x1 - 1) + (j - A.y1 - 1) + (k - A.z1 - 1)) % (A.x2 - A.x1)) * (ny * nz) +
+                      (j - A.y1 - 1) + ny * (k - A.z1 - 1);
   A.Q[w] = q;
   A.S[w] = s;
 }
 
-// One D_T: the planes in order.  Column (j, k) of plane s holds i = s − j − k, so the old θ of i+1, j+1 and k+1 are in
-// plane s + 1 (columns c, c + 1, c + ny) and the new θ of i−1, j−1 and k−1 in plane s − 1 (c, c − 1, c − ny); beyond
-// the block's inner nodes each is the node's own old θ (the face's copy).  P2: the squared spacings are powers of two,
-// so a product by the reciprocal is the quotient's bits and the chain holds one division instead of two.
+// One D_T: the planes in order.  Plane s takes the slot s mod nx: a column (j, k) has its nx nodes in as many successive
+// planes, so each node has its own entry and the arrays are as large as the block, whatever its shape.  Column (j, k) of
+// plane s holds i = s − j − k, so the old θ of i+1, j+1 and k+1 are in plane s + 1 (columns c, c + 1, c + ny) and the new
+// θ of i−1, j−1 and k−1 in plane s − 1 (c, c − 1, c − ny); beyond the block's inner nodes each is the node's own old θ
+// (the face's copy).  P2: the squared spacings are powers of two, so a product by the reciprocal is the quotient's bits
+// and the chain holds one division instead of two.
 template <bool P2>
 __global__ void __launch_bounds__(HT_THREADS) k_heat_sweep(const __grid_constant__ HeatArgs A) {
   extern __shared__ double hsh[];
@@ -156,23 +159,25 @@ __global__ void __launch_bounds__(HT_THREADS) k_heat_sweep(const __grid_constant
   const double rx = 1 / A.dx2, ry = 1 / A.dy2, rz = 1 / A.dz2;
   auto div = [](double v, double d, double r) { return P2 ? v * r : v / d; };
   const int ns = nx + ny + nz - 2;
-  for (int s = 0; s < ns; s++) {
+  for (int s = 0, m = 0; s < ns; s++) {   // m = s mod nx
+    const int mn = m + 1 < nx ? m + 1 : 0;
     const double *pv = buf + ((s + 1) & 1) * nc;
     double *nw = buf + (s & 1) * nc;
     for (int c = threadIdx.x; c < nc; c += blockDim.x) {
       const int k = c / ny, j = c - k * ny, i = s - j - k;
       if (i < 0 || i >= nx) continue;
-      double *Qs = A.Q + (long long)s * nc + c;
-      const double *Qn = Qs + nc;
+      double *Qs = A.Q + (long long)m * nc + c;
+      const double *Qn = A.Q + (long long)mn * nc + c;
       const double q = Qs[0];
       const double xp = i + 1 < nx ? Qn[0] : q, yp = j + 1 < ny ? Qn[1] : q, zp = k + 1 < nz ? Qn[ny] : q;
-      const double src = A.S[(long long)s * nc + c];
+      const double src = A.S[(long long)m * nc + c];
       const double xm = i > 0 ? pv[c] : q, ym = j > 0 ? pv[c - 1] : q, zm = k > 0 ? pv[c - ny] : q;
       const double flux = A.DT * (div((xp - 2 * q) + xm, A.dx2, rx) + div((yp - 2 * q) + ym, A.dy2, ry) + div((zp - 2 * q) + zm, A.dz2, rz));
       const double tn = heat_node(A, q, flux, src);
       nw[c] = tn;
       Qs[0] = tn;
     }
+    m = mn;
     __syncthreads();
   }
 }
@@ -186,7 +191,7 @@ __global__ void __launch_bounds__(HT_BS) k_heat_store(const __grid_constant__ He
   const int i = (int)(u - b * (unsigned)nx), j = (int)(b - k * (unsigned)ny);
   const long long o = A.d.at(A.x1 + 1 + i, A.y1 + 1 + j, A.z1 + 1 + (int)k);
   if (A.uni) {
-    A.T[o] = A.Q[(long long)(i + j + (int)k) * (ny * nz) + j + ny * (int)k];
+    A.T[o] = A.Q[(long long)((i + j + (int)k) % nx) * (ny * nz) + j + ny * (int)k];
     return;
   }
   const long long sx = 1, sy = A.d.n1, sz = (long long)A.d.n1 * A.d.n2;
@@ -232,7 +237,7 @@ int heat_create(Ctx *ctx, const tdgl_materials *M) {
   // not fit shared memory
   const Geo &g = ctx->g;
   const size_t nc = (size_t)(g.y2 - g.y1) * (g.z2 - g.z1);
-  const size_t np = (size_t)((g.x2 - g.x1) + (g.y2 - g.y1) + (g.z2 - g.z1) - 2) * nc;
+  const size_t np = (size_t)(g.x2 - g.x1) * nc;
   if ((rc = dalloc(ctx, &ctx->heat_S, ctx->Th2 ? (size_t)nn : np))) return rc;
   if (!ctx->Th2 && (rc = dalloc(ctx, &ctx->heat_Q, np))) return rc;
   if (!ctx->Th2 && 2 * nc * sizeof(double) > HT_SMEM && (rc = dalloc(ctx, &ctx->heat_prev, 2 * nc))) return rc;
