@@ -560,6 +560,13 @@ int tdgl_ctx_create(const tdgl_params *p, tdgl_ctx **out) {
     if ((e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess) return fail(set_err(ctx, TDGL_ECUDA, "drag", e));
   }
   if (p->vac) {   // node-shaped already: a plain copy
+    for (int k = g.z1; k <= g.z2 + 1; k++)
+      for (int j = g.y1; j <= g.y2 + 1; j++)
+        for (int i = g.x1; i <= g.x2 + 1; i++) {   // (an inner node copies itself)
+          const int ii = std::min(std::max(i, g.x1 + 1), g.x2), jj = std::min(std::max(j, g.y1 + 1), g.y2),
+                    kk = std::min(std::max(k, g.z1 + 1), g.z2);
+          ctx->vac_late = ctx->vac_late || (p->vac[g.d.at(ii, jj, kk)] && !p->vac[g.d.at(i, j, k)]);
+        }
     if ((rc = dalloc(ctx, &ctx->vac, (size_t)nn))) return fail(rc);
     if ((e = cudaMemcpyAsync(ctx->vac, p->vac, (size_t)nn, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
       return fail(set_err(ctx, TDGL_ECUDA, "vacuum map upload", e));

@@ -266,6 +266,7 @@ struct Ctx {
   MatDev *mt = nullptr;
   bool haskwt_mat[TDGL_MAXB] = {};   // KWT on band µ in some material
   uint8_t *vac = nullptr;            // a sculpted sample: nonzero on the vacuum nodes (null: no vacuum)
+  bool vac_late = false;             // a node of the block's shell is no vacuum, the node inside that it copies is
   // per-step values: the device copy the kernels read, and the pinned host slots of the current call
   StepScal *ss_cur = nullptr;
   StepScal *ss_host = nullptr;

@@ -115,7 +115,10 @@ __device__ __forceinline__ void scale_b(const Blk bk, ScaleArgs const &A) {
 // ends): links U = e^{−iφ} (0..2), the curl on the inner plaquettes (3..5), the outer faces of h (6..14: per
 // component the k faces, the j faces and the i faces), the block's nodes of every band (15).  No item reads what
 // another writes: the faces of h are disjoint from the plaquettes of the curl, the ghosts take their links from φ
-// (the same e^{−iφ}) and read nodes inside the block, which no item writes in F.
+// (the same e^{−iφ}) and read nodes inside the block, which no item writes in F but to clear vacuum.  A vacuum node may
+// hold Ψ ≠ 0 until the first step of an uploaded state has ended (an RKL/RKC combination keeps its share of it), so a
+// ghost beside one could be formed before or after it is cleared: it does not matter where the ghost is vacuum too, as
+// `sculpt` makes it; a sample with another ghost beside vacuum (vac_late) is cleared by a launch of its own afterwards.
 // What bounds it: an FP64 sincos per link on large grids; on small ones it is one launch where the links with the
 // curl, the faces of h, the ghosts of each band and the copy of advance! were N + 3, each waiting for the one before.
 // 40 steps took 2709 µs instead of 2811 (12×8×4 cells), 3597 instead of 3782 (64×32×8), 7638 instead of 7893
@@ -140,6 +143,7 @@ struct FinArgs {
   int N;
   int x1, x2, y1, y2, z1, z2;
   const uint8_t *vac;       // a sculpted sample: F = 0 on every vacuum node (range 15 is then the whole grid)
+  int vac_late;             // leave F on the vacuum inside the block as it is (k_vacuum_zero follows)
 };
 
 // advance! alone, for blocks one cell thick
@@ -342,7 +346,7 @@ __device__ __forceinline__ void finish_b(const Blk bk, FinArgs const &A) {
     }
     const bool vac = A.vac && A.vac[o];
     for (int mu = 0; mu < A.N; mu++) {
-      if (vac) A.F[mu][o] = mkc(0.0, 0.0);
+      if (vac && !A.vac_late) A.F[mu][o] = mkc(0.0, 0.0);
       if (block) A.G[mu][o] = vac ? mkc(0.0, 0.0) : A.F[mu][o];   // outside the block: with vacuum only
     }
   }
@@ -378,6 +382,7 @@ void finish_step(Ctx *ctx) {
   A.N = ctx->N;
   A.x1 = g.x1; A.x2 = g.x2; A.y1 = g.y1; A.y2 = g.y2; A.z1 = g.z1; A.z2 = g.z2;
   A.vac = ctx->vac;
+  A.vac_late = ctx->vac_late;
   // a block one cell thick has no node inside: its face passes read each other's ghosts and run one after the other
   const bool thin = g.x2 < g.x1 + 1 || g.y2 < g.y1 + 1 || g.z2 < g.z1 + 1;
   A.r[15] = ctx->vac ? mkrng(1, g.Nx + 1, 1, g.Ny + 1, 1, g.Nz + 1) : mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
@@ -388,6 +393,7 @@ void finish_step(Ctx *ctx) {
   const double nl = (double)A.off[3], nh = (double)(A.off[6] - A.off[3]), nf = (double)(A.off[15] - A.off[6]);
   const double bytes = 24.0 * nl + 8.0 * nh + (A.open ? 32.0 : 16.0) * nf + 32.0 * ctx->N * A.r[15].n();
   TDGL_LAUNCH(ctx, K_LINKSCURL, bytes, k_finish, nblk(A.off[16], BS), BS, 0, A);
+  if (ctx->vac_late && !thin) vacuum_zero(ctx);
   if (thin) {
     for (int mu = 0; mu < ctx->N; mu++) ghosts(ctx, ctx->F[mu], ctx->U[0], ctx->U[1], ctx->U[2]);
     if (ctx->vac) vacuum_zero(ctx);
