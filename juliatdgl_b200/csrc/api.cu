@@ -22,12 +22,12 @@ int set_err(Ctx *ctx, int code, const char *what, cudaError_t e) {
 }
 
 const char *kcat_name[K_NCAT] = {"band_stage", "link_rotation", "neumann_ghosts", "frame_rate_faces", "current_increment",
-                                  "links_curl", "face_field", "advance", "scale_increment", "sep_transform_f64",
+                                  "links_curl", "scale_increment", "sep_transform_f64",
                                   "sep_modes_f64", "precond_transform_f32", "precond_modes_f32", "precond_convert",
-                                  "pcg_start", "pcg_curl", "pcg_apply", "pcg_residual", "pcg_update", "pcg_dot",
-                                  "pcg_final", "pcg_direction", "pcg_extrap", "pack", "open_fft", "open_misc", "copy",
+                                  "pcg_apply", "pcg_residual", "pcg_update", "pcg_dot",
+                                  "pcg_final", "pcg_extrap", "pack", "open_fft", "open_misc", "copy",
                                   "meter", "noise", "precond_inverse_f32", "heat", "pcg_update_x",
-                                  "pcg_dot_side", "qp_exchange"};
+                                  "qp_exchange"};
 
 cudaEvent_t prof_begin(Ctx *ctx) {
   Prof &p = ctx->prof;

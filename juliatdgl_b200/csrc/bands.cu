@@ -255,29 +255,6 @@ __device__ __forceinline__ void band_stage_b(const Blk bk, StageArgs const &A) {
   A.C[o] = v;
 }
 
-// Covariant Neumann ghosts of one band on one pair of faces (bands.jl:524-539), for blocks one cell thick (see
-// finish_step, field.cu).
-__device__ __forceinline__ void ghost_face_b(const Blk bk, cd * const &X, const cd * const &Lk, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi);
-__global__ void k_ghost_face(cd *X, const cd *Lk, Dim d, Rng r, int axis, int lo, int hi) { ghost_face_b(TDGL_BLK, X, Lk, d, r, axis, lo, hi); }
-TDGL_MERGEABLE(k_ghost_face, ghost_face_b, 256, 1, false);
-__device__ __forceinline__ void ghost_face_b(const Blk bk, cd * const &X, const cd * const &Lk, Dim const &d, Rng const &r, int const &axis, int const &lo, int const &hi) {
-  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
-  if (t >= r.n()) return;
-  int a, b, c;
-  rng_ijk(r, t, a, b, c);
-  auto L = [&](long long q) { return Lk[q]; };
-  if (axis == 0) {
-    X[d.at(lo, b, c)] = cmul(L(d.at(lo, b, c)), X[d.at(lo + 1, b, c)]);
-    X[d.at(hi + 1, b, c)] = cmul(cconj(L(d.at(hi, b, c))), X[d.at(hi, b, c)]);
-  } else if (axis == 1) {
-    X[d.at(a, lo, c)] = cmul(L(d.at(a, lo, c)), X[d.at(a, lo + 1, c)]);
-    X[d.at(a, hi + 1, c)] = cmul(cconj(L(d.at(a, hi, c))), X[d.at(a, hi, c)]);
-  } else {
-    X[d.at(a, b, lo)] = cmul(L(d.at(a, b, lo)), X[d.at(a, b, lo + 1)]);
-    X[d.at(a, b, hi + 1)] = cmul(cconj(L(d.at(a, b, hi))), X[d.at(a, b, hi)]);
-  }
-}
-
 // Link operations over the three link ranges of the band stencil (_rx, _ry, _rz, bands.jl:349-351).
 enum LinkOp { LOP_ROT_INIT = 0, LOP_ADVANCE, LOP_FRAME_LINKS, LOP_LINK_RATE };
 
@@ -590,16 +567,6 @@ void clear_outside(Ctx *ctx) {
       k_zero_outside<<<nblk(n, BS), BS, 0, ctx->stream>>>(ctx->F[mu], ctx->g);
       ctx->launches++;
     }
-}
-
-void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz) {
-  const Geo &g = ctx->g;
-  Rng r0 = mkrng(1, 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
-  Rng r1 = mkrng(g.x1, g.x2 + 1, 1, 1, g.z1, g.z2 + 1);
-  Rng r2 = mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, 1, 1);
-  TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r0.n(), k_ghost_face, nblk(r0.n(), BS), BS, 0, X, Lx, g.d, r0, 0, g.x1, g.x2);
-  TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r1.n(), k_ghost_face, nblk(r1.n(), BS), BS, 0, X, Ly, g.d, r1, 1, g.y1, g.y2);
-  TDGL_LAUNCH(ctx, K_GHOST, 96.0 * r2.n(), k_ghost_face, nblk(r2.n(), BS), BS, 0, X, Lz, g.d, r2, 2, g.z1, g.z2);
 }
 
 struct BandOut {

@@ -142,9 +142,9 @@ namespace tdgl {
 // Kernel categories of the per-launch profiler (tdgl_profile): CUDA events around every launch, with the
 // algorithmic (compulsory) bytes of that launch, so that a driver can report achieved bandwidth per kernel.
 enum KCat {
-  K_BAND = 0, K_LINK, K_GHOST, K_OMEGA, K_CURINC, K_LINKSCURL, K_FACEH, K_ADVANCE, K_SCALE, K_TX64, K_MODES64,
-  K_TX32, K_MODES32, K_CONVERT, K_PCG_START, K_PCG_H, K_PCG_Q, K_PCG_RES, K_PCG_UPD, K_PCG_DOT, K_PCG_FINAL,
-  K_PCG_DIR, K_PCG_EXTRAP, K_PACK, K_OPEN_FFT, K_OPEN_MISC, K_COPY, K_METER, K_NOISE, K_TX32I, K_HEAT, K_PCG_XUPD, K_PCG_DOTS, K_QP, K_NCAT
+  K_BAND = 0, K_LINK, K_GHOST, K_OMEGA, K_CURINC, K_LINKSCURL, K_SCALE, K_TX64, K_MODES64,
+  K_TX32, K_MODES32, K_CONVERT, K_PCG_Q, K_PCG_RES, K_PCG_UPD, K_PCG_DOT, K_PCG_FINAL,
+  K_PCG_EXTRAP, K_PACK, K_OPEN_FFT, K_OPEN_MISC, K_COPY, K_METER, K_NOISE, K_TX32I, K_HEAT, K_PCG_XUPD, K_QP, K_NCAT
 };
 extern const char *kcat_name[K_NCAT];
 
@@ -403,7 +403,6 @@ void field_kick(Ctx *ctx);
 // bands.cu
 int update_bands(Ctx *ctx);
 void clear_outside(Ctx *ctx);   // F = 0 outside the block, once for a state that came in from outside
-void ghosts(Ctx *ctx, cd *X, const cd *Lx, const cd *Ly, const cd *Lz);
 void vacuum_zero(Ctx *ctx);   // neumann! on a sculpted sample: F = 0 on every vacuum node
 // field.cu
 void supercurrent_increment(Ctx *ctx);

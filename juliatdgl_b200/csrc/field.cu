@@ -146,27 +146,6 @@ struct FinArgs {
   int vac_late;             // leave F on the vacuum inside the block as it is (k_vacuum_zero follows)
 };
 
-// advance! alone, for blocks one cell thick
-struct AdvArgs {
-  cd *G[TDGL_MAXB];
-  const cd *F[TDGL_MAXB];
-  int N;
-  Rng r;
-  Dim d;
-};
-
-__device__ __forceinline__ void advance_b(const Blk bk, AdvArgs const &A);
-__global__ void k_advance(AdvArgs A) { advance_b(TDGL_BLK, A); }
-TDGL_MERGEABLE(k_advance, advance_b, BS, 1, false);
-__device__ __forceinline__ void advance_b(const Blk bk, AdvArgs const &A) {
-  long long t = (long long)bk.x * blockDim.x + threadIdx.x;
-  if (t >= A.r.n()) return;
-  int i, j, k;
-  rng_ijk(A.r, t, i, j, k);
-  const long long o = A.d.at(i, j, k);
-  for (int mu = 0; mu < A.N; mu++) A.G[mu][o] = A.F[mu][o];
-}
-
 // Shell of a box (a, b, c) split into k faces, j faces and i faces without overlap.
 void shell(int a, int b, int c, Rng *r) {
   r[0] = mkrng(1, a, 1, b, 1, 1);
@@ -383,30 +362,14 @@ void finish_step(Ctx *ctx) {
   A.x1 = g.x1; A.x2 = g.x2; A.y1 = g.y1; A.y2 = g.y2; A.z1 = g.z1; A.z2 = g.z2;
   A.vac = ctx->vac;
   A.vac_late = ctx->vac_late;
-  // a block one cell thick has no node inside: its face passes read each other's ghosts and run one after the other
-  const bool thin = g.x2 < g.x1 + 1 || g.y2 < g.y1 + 1 || g.z2 < g.z1 + 1;
   A.r[15] = ctx->vac ? mkrng(1, g.Nx + 1, 1, g.Ny + 1, 1, g.Nz + 1) : mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
-  if (thin) A.r[15].ni = 0;
   A.off[0] = 0;
   for (int q = 0; q < 16; q++) A.off[q + 1] = A.off[q] + A.r[q].n();
   A.d = g.d;
   const double nl = (double)A.off[3], nh = (double)(A.off[6] - A.off[3]), nf = (double)(A.off[15] - A.off[6]);
   const double bytes = 24.0 * nl + 8.0 * nh + (A.open ? 32.0 : 16.0) * nf + 32.0 * ctx->N * A.r[15].n();
   TDGL_LAUNCH(ctx, K_LINKSCURL, bytes, k_finish, nblk(A.off[16], BS), BS, 0, A);
-  if (ctx->vac_late && !thin) vacuum_zero(ctx);
-  if (thin) {
-    for (int mu = 0; mu < ctx->N; mu++) ghosts(ctx, ctx->F[mu], ctx->U[0], ctx->U[1], ctx->U[2]);
-    if (ctx->vac) vacuum_zero(ctx);
-    AdvArgs V;
-    for (int mu = 0; mu < ctx->N; mu++) {
-      V.G[mu] = ctx->G[mu];
-      V.F[mu] = ctx->F[mu];
-    }
-    V.N = ctx->N;
-    V.r = mkrng(g.x1, g.x2 + 1, g.y1, g.y2 + 1, g.z1, g.z2 + 1);
-    V.d = g.d;
-    TDGL_LAUNCH(ctx, K_ADVANCE, 32.0 * ctx->N * V.r.n(), k_advance, nblk(V.r.n(), BS), BS, 0, V);
-  }
+  if (ctx->vac_late) vacuum_zero(ctx);
   advance_swap(ctx);
 }
 

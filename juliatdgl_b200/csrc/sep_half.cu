@@ -28,7 +28,7 @@ namespace {
 // of 111.  Before, each component and class had its own launch of 48 × 96 tiles without prefetching: 36 launches of
 // 25 µs per PCG iteration there, two blocks per SM each.
 enum HMode { ROW_F, ROW_I, COL_F, COL_I };
-const int HG_N = 128, HG_K = 16, HG_ST = 3, HG_WS = 64, HG_DS = HG_N + 12, HG_MAXT = 128;
+const int HG_N = 128, HG_K = 16, HG_ST = 3, HG_WS = 64, HG_DS = HG_N + 12;
 
 struct HGroup {
   const float *W;   // [K][ldw], columns beyond the block zero up to ldw (a multiple of 8)
