@@ -287,7 +287,9 @@ __global__ void __launch_bounds__(AP_T, 2) k_apply(const __grid_constant__ Apply
 }
 
 // The distinct values of the conductivities as a table of at most 256, and each entry's place in it: an open-addressed
-// set of bit patterns (a value takes its hash's slot or a later one).  *bad counts the entries that found no place.
+// set of bit patterns (a value takes its hash's slot or a later one).  The first pass (no codes) fills the set and stops
+// once a value found no place (*bad): with more values than places every further link would walk the whole set for
+// nothing.  The second, when all have one, writes the codes.
 const unsigned long long DT_FREE = 0xfff8dead0000beefULL;   // no value a conductivity has (a NaN with this payload)
 __global__ void k_dtab_clear(unsigned long long *tab, int *bad) {
   tdgl::pdl_enter();
@@ -297,7 +299,7 @@ __global__ void k_dtab_clear(unsigned long long *tab, int *bad) {
 __global__ void k_dtab(CVec3 D, long long n, unsigned long long *tab, uint8_t *c0, uint8_t *c1, uint8_t *c2, int *bad) {
   tdgl::pdl_enter();
   uint8_t *code[3] = {c0, c1, c2};
-  for (int c = 0; c < 3; c++)
+  for (int c = 0; c < 3 && !*(volatile int *)bad; c++)
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
       const unsigned long long v = (unsigned long long)__double_as_longlong(D.p[c][t]);
       unsigned h = (unsigned)((v ^ (v >> 29) ^ (v >> 47)) * 0x9e3779b1u) >> 24;
@@ -307,8 +309,12 @@ __global__ void k_dtab(CVec3 D, long long n, unsigned long long *tab, uint8_t *c
         if (w == DT_FREE) w = atomicCAS(tab + h, DT_FREE, v);
         if (w == DT_FREE || w == v) break;
       }
-      if (left == 0 || v == DT_FREE) atomicAdd(bad, 1);
-      code[c][t] = (uint8_t)h;
+      if (left == 0 || v == DT_FREE) {
+        *(volatile int *)bad = 1;
+        return;
+      }
+      if (c0) code[c][t] = (uint8_t)h;
+      else if (*(volatile int *)bad) return;
     }
 }
 
@@ -591,17 +597,20 @@ int pcg_create(Ctx *ctx) {
   const double *D[3] = {ctx->D[0], ctx->D[1], ctx->D[2]};
   to_planes(ctx, D, nullptr, S->Dp);
   // as byte codes where they have at most 256 values
-  for (int c = 0; c < 3; c++)
-    if ((rc = dalloc(ctx, &S->Dc[c], S->n))) return rc;
   if ((rc = dalloc(ctx, &S->Dt, 256))) return rc;
   CVec3 dv = cv(S->Dp);
   k_dtab_clear<<<1, 256, 0, ctx->stream>>>((unsigned long long *)S->Dt, S->ic);
-  k_dtab<<<S->sblocks, BS, 0, ctx->stream>>>(dv, S->n, (unsigned long long *)S->Dt, S->Dc[0], S->Dc[1], S->Dc[2], S->ic);
+  k_dtab<<<S->sblocks, BS, 0, ctx->stream>>>(dv, S->n, (unsigned long long *)S->Dt, nullptr, nullptr, nullptr, S->ic);
   int bad = 0;
   TDGL_CUDA(cudaMemcpyAsync(&bad, S->ic, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   TDGL_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (bad)
-    for (int c = 0; c < 3; c++) S->Dc[c] = nullptr;
+  if (bad) return 0;
+  uint8_t *code[3];
+  for (int c = 0; c < 3; c++)
+    if ((rc = dalloc(ctx, &code[c], S->n))) return rc;
+  k_dtab<<<S->sblocks, BS, 0, ctx->stream>>>(dv, S->n, (unsigned long long *)S->Dt, code[0], code[1], code[2], S->ic);
+  for (int c = 0; c < 3; c++) S->Dc[c] = code[c];
+  TDGL_CUDA(cudaGetLastError());
   return 0;
 }
 
