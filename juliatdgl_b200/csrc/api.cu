@@ -998,7 +998,10 @@ static int batch_capture(tdgl_batch_impl *b, int k) {
     for (int i = 0; i < nc; i++) b->par0[i] = b->c[i]->parity;
   }
   b->glaunch[k].assign(nc, 0);
-  b->tape[k].assign(nc, Tape());
+  Tape blank;
+  for (Ctx *ctx : b->c)
+    if (ctx->P.solver == TDGL_SOLVER_SEP) blank.planes += ctx->g.Nx - 1;
+  b->tape[k].assign(nc, blank);
   b->added[k].assign(nc, {});
   cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return set_err(c0, TDGL_ECUDA, "batch capture", e);

@@ -217,6 +217,7 @@ struct TapeRec {
 };
 struct Tape {
   bool ok = true;
+  long long planes = 0;   // x-planes of the separable solves of all contexts of the batch
   std::vector<TapeRec> recs;
 };
 

@@ -88,7 +88,7 @@ struct PlaneMulti {
   PlaneArgs c[3];
 };
 
-const int PL_JC = 48, PL_THREADS = 192, PL_PPB = 8;
+const int PL_JC = 48, PL_THREADS = 192, PL_PPB = 8, PL_WHOLE = 6;
 
 __device__ __forceinline__ void ld4(float *v, const float *p) {
   const float4 t = *reinterpret_cast<const float4 *>(p);
@@ -1282,15 +1282,21 @@ void plane(Ctx *ctx, PlaneMulti M) {
     // several planes (a merged launch gives each context fewer blocks); persistent: a block keeps its basis chunks
     // in shared memory for all its planes (about four blocks per SM a component).  Small planes take 2-row tiles.
     // A run alone has rows to spare for few SMs: chunks of at most PL_JC rows (192×64×16 cells: 6539 µs a cycle; with
-    // one chunk 6918).  A step that a batch records fills the GPU with its other runs' planes: whole planes of at most
-    // 2 PL_JC rows, whose input and second basis are then loaded once (16 runs: 34.5 → 32.1 ms a cycle; the same bits).
+    // one chunk 6918).  A batch with at least PL_WHOLE planes per SM fills the GPU: whole planes of at most 2 PL_JC rows,
+    // whose input and second basis are then loaded once.  Below, a merged launch has so few planes a block that whole
+    // ones end it raggedly.  Whole planes against chunks, a cycle of batches of three draws of the sweep (the same
+    // bits): 16 runs (1872 to 2096 planes) 30.4 to 33.7 ms against 31.6 to 36.0; 8 runs, 15.2 against 15.7 (968
+    // planes), 19.7 against 20.0 (1160), but 15.7 against 15.2 (872); 6 runs (646 to 838) 11.1 to 15.2 against 10.8 to
+    // 14.7; 4 runs (324 to 548) 8.3 to 11.5 against 7.4 to 11.0; 3 runs (259 to 483) 5.6 to 11.0 against 5.4 to 9.9; 2 runs
+    // (162 to 386) either way by 5 %.
     const bool small = njm <= 2 * PL_JC;
     const int nsm = g_sm_count > 0 ? g_sm_count : 148;
+    const bool whole = small && ctx->tape && ctx->tape->planes >= (long long)PL_WHOLE * nsm;
     size_t smem = 0;
     int ngy = 1, gx = 1;
     for (int c = 0; c < 3; c++) {
       PlaneArgs &A = M.c[c];
-      const int rows = small && ctx->tape ? 2 * PL_JC : PL_JC, ny = (A.nj_out + rows - 1) / rows;
+      const int rows = whole ? 2 * PL_JC : PL_JC, ny = (A.nj_out + rows - 1) / rows;
       A.jc = small ? rup4((A.nj_out + ny - 1) / ny) : PL_JC;
       const int ta = small ? 2 : 4;
       const int tiles = (A.jc / ta) * (std::max(rup4(A.nk_in), rup4(A.nk_out)) / 4);
