@@ -1067,9 +1067,10 @@ void linesolve(Ctx *ctx, SepDev *S, Work<T> &w, const int *done) {
   const long long P = S->P;
   const KCat cat = sizeof(T) == 8 ? K_MODES64 : K_MODES32;
   const double bytes = (6.0 * sizeof(T) + 8.0) * nx * P;   // X, Y, Z in and out; the factorisation in
-  // a step that a batch records takes the staged kernel: its chunks have one form for every length, so runs of different
-  // lengths share a merged launch (the same bits)
-  const auto warp = ctx->tape ? nullptr : linesolve_warp_kernel<T>(nx);
+  // a step that a batch may merge takes the staged kernel: its chunks have one form for every length, so runs of
+  // different lengths share a merged launch (the same bits); a PCG's loop is never merged
+  const bool merges = ctx->tape && ctx->P.solver == TDGL_SOLVER_SEP;
+  const auto warp = merges ? nullptr : linesolve_warp_kernel<T>(nx);
   if (warp) {
     TDGL_LAUNCH(ctx, cat, bytes, warp, (int)((P + LS2_LINES - 1) / LS2_LINES), LS2_THREADS, ls3_smem<T>(nx), w.Xh, w.Yh, w.Zh, w.inv, nx,
                 P, S->ny, S->bd[1].s, S->bd[2].s, ctx->P.a_imp, done);

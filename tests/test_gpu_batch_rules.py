@@ -1,9 +1,11 @@
 """Batches on either side of the rules that a recorded step follows: planes of 49 to 96 rows in row chunks (few planes in
-flight) and whole (many), each run with the bits it has alone."""
+flight) and whole (many), and PCG runs on lines of several nodes a lane (their loops never merge) beside runs that do;
+each run with the bits it has alone."""
 import numpy as np
 import pytest
 
 import cases
+import juliatdgl_b200 as T
 from juliatdgl_b200 import gpu
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +54,16 @@ def test_many_planes_in_flight():
     runs = [cases.small("rkl_bar", grid=g) for g in grids]
     assert sum(r[0].grid.Nx - 1 for r in runs) >= 6 * 148
     _check(runs, 6, 4)
+
+
+def _pcg(nx, f32):
+    gr = T.Grid.make(nx, 8, 4, dx=0.5, buf=2)
+    md = T.two_band(xi_ratio=4.0, κ=2.0, gamma_kwt=10.0)
+    st = T.Stepper.make(md, gr, T.box_masks(gr), σvac=0.01, pcg_tol=1e-10, pcg_f32=f32)
+    return st, T.initial_state(md, gr, st.masks, 0.03), 0.03, T.selffield(st, 0.3)
+
+
+def test_pcg_runs_on_long_lines():
+    runs = [_pcg(64, True), _pcg(150, False), _pcg(230, True)]
+    runs += [cases.small("rkl_bar", grid=g) for g in ((90, 8, 4), (40, 10, 5))]
+    _check(runs, 10, 2)
