@@ -168,10 +168,10 @@ class Clocks:
 
 
 # ---------------------------------------------------------------------------------------------- arms
-# DRAM bytes (read + write) per launch of the kernels of ramp256, one `ncu --set full --clock-control none` capture
-# per kernel of `python bench.py --quick --no-graphs --steps 1 --warmup 1` (summaries under profiles/): the
-# roofline's `traffic`, to set against the algorithmic bytes the live run measures.
-NCU_TRAFFIC = {"precond_transform_f32": 22.24e6, "open_fft": 482.8e6}
+# DRAM bytes (read + write) per launch of the kernels of ramp256, from ncu with `--clock-control none` (a step's mean for
+# the band stages; summaries under profiles/): the roofline's `traffic`, to set against the algorithmic bytes the live
+# run measures.
+NCU_TRAFFIC = {"precond_transform_f32": 22.1e6, "pcg_apply": 118.1e6, "band_stage": 160.4e6, "open_fft": 482.8e6}
 FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12   # SMs × FP32 lanes × 2 × max SM clock
 
 

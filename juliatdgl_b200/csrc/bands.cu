@@ -6,8 +6,8 @@
 // combination (_combine! :425-430) and the final turn back (_frame_turn! :321-327).  The links of later RKL/RKC stages
 // (_rotlinks!, _rotfrac!) are formed where a stage reads them; the other link rotations (_rot!, _advance_links!,
 // _frame_links!, _link_rate!, :292-423) run as one kernel over the three link ranges.  The covariant Neumann ghosts of
-// an intermediate stage (ghosts! :524-539) are formed in the next stage too, the step's final ones by one pass over the
-// block's shell.
+// an intermediate stage (ghosts! :524-539) are formed in the next stage too, the step's final ones at the end of the
+// step (k_finish, field.cu).
 #include "common.cuh"
 #include "merge.cuh"
 

@@ -323,11 +323,11 @@ void tape_record(Ctx *ctx, void (*kern)(P...), dim3 grid, dim3 block, size_t sme
 // A launch whose blocks may become resident while the kernel before it in the stream drains: every kernel that is
 // launched so begins with pdl_enter(), which waits for that kernel to finish before it touches memory, so the order of
 // the work is that of plain launches.  What it hides is the launch latency between two kernels of the solvers' loops
-// (pcg.cu, qp.cu and the preconditioner's transforms), at most two blocks per SM: 40 steps 63.8 → 61.3 ms (two fluids,
-// 40×20×8 cells), 18.7 → 18.2 (the ramp, 64×32×8), 229.3 → 223.1 (256×128×32).  Larger grids gain nothing, and the
+// (pcg.cu, qp.cu and the preconditioner's transforms), at most two blocks per SM: 40 steps 63.0 → 59.4 ms (two fluids,
+// 40×20×8 cells), 19.1 → 17.5 (the ramp, 64×32×8), 225.4 → 220.5 (256×128×32).  Larger grids gain nothing, and the
 // kernels outside the loops lose (192×64×16 without padding: 6514 → 6838 µs): blocks that wait early keep the bands'
 // parallel branches off the SMs, and those of a wide kernel gather on the SMs that drain first.
-const long long EARLY_BLOCKS = 296;
+const long long EARLY_BLOCKS = 2 * 148;   // two on each of a B200's SMs
 template <class... P, class... A>
 void launch_kernel(Ctx *ctx, bool early, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, A &&...a) {
   cudaLaunchConfig_t c = {};

@@ -119,7 +119,8 @@ __device__ __forceinline__ void scale_b(const Blk bk, ScaleArgs const &A) {
 // hold Ψ ≠ 0 until the first step of an uploaded state has ended (an RKL/RKC combination keeps its share of it), so a
 // ghost beside one could be formed before or after it is cleared: it does not matter where the ghost is vacuum too, as
 // `sculpt` makes it; a sample with another ghost beside vacuum (vac_late) is cleared by a launch of its own afterwards.
-// What bounds it: an FP64 sincos per link on large grids; on small ones it is one launch where the links with the
+// What bounds it on large grids: issue (63 %) and the latency of its loads (2.4 TB/s; the FP64 pipe, with a sincos per
+// link, is at 10 %); on small ones it is one launch where the links with the
 // curl, the faces of h, the ghosts of each band and the copy of advance! were N + 3, each waiting for the one before.
 // 40 steps took 2709 µs instead of 2811 (12×8×4 cells), 3597 instead of 3782 (64×32×8), 7638 instead of 7893
 // (192×64×16), 245.9 ms instead of 250.0 (the 256×128×32 ramp).  The registers are held to 40: with the

@@ -11,7 +11,7 @@
 // before in shared memory, and k_heat_store brings the result back.  What bounds the sweep is the latency of a plane:
 // a block barrier, a shared load and the FP64 chain with a division.  When one block also computed the sources and
 // read the grid's own arrays (a sector per thread and load), the heat model took 574 µs of a 683 µs step on 96×48×8
-// cells; a step there takes 226 µs now.
+// cells; a step there takes 215 µs now.
 #include <algorithm>
 #include <cmath>
 

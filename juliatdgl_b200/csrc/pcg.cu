@@ -7,8 +7,8 @@
 //
 // Iterates, residuals and dot products are FP64; z is held in the precision the preconditioner computes it in.  Every
 // vector is a plane-major node-shaped array per component (sep.cu), zero outside the ranges, so the vector kernels are
-// flat loops.  A·p forms the new direction p = z + βp and the curl of p on the fly (no plaquette arrays).  Dot products are deterministic: a fixed grid of block partial sums reduced by one block
-// in a fixed order.  The loop runs on the device: α, β and the convergence test (‖r‖ ≤ tol·‖b‖) are computed by
+// flat loops.  A·p forms the new direction p = z + βp and the curl of p on the fly (no plaquette arrays).  Dot products
+// are deterministic: a fixed grid of block partial sums reduced by one block in a fixed order.  The loop runs on the device: α, β and the convergence test (‖r‖ ≤ tol·‖b‖) are computed by
 // the reduction kernels, and once the test passes every later kernel of the iteration returns at once; the host
 // launches iterations in batches and reads the flag between batches only.
 #include <algorithm>
@@ -97,16 +97,17 @@ __global__ void __launch_bounds__(256, 8) k_dot2(CVec3 a, ZVec3<T> b, ZVec3<T> c
 // partial sums of P·Q, over the box i ∈ 2..Nx, j ∈ 2..Ny, k ∈ 2..Nz.  With DIR the direction is formed here too,
 // P = z + βP (the solve's first iteration, ic[IC_ITERS] = 0: P = z), from the old P into the other buffer.
 //
-// What bounds it: HBM.  A block takes a tile of tj × tk columns (tj ≤ 24 rows of the unit-stride axis; both split
-// evenly), a column per thread, and marches over `chunk` planes i.  A thread reads its own column (and one element of
-// the tile's halo) straight into registers two planes ahead, forms P, and leaves it in shared memory for its
-// neighbours: three planes in turn, so that one barrier a plane suffices.  The plaquettes of plane i − 1 that plane i
-// needs are the thread's own, kept in registers.  Each plane is read once per tile with a halo of one row and column.
-// The conductivities are a byte per link where they have at most 256 values (padding, materials), looked up in shared
-// memory.  One thread per node reading its 36 neighbours through L1 fetched each plane several times from L2, and the
-// direction was a pass of its own: 57 + 24 µs on the 256×128×32 ramp, 78 + 31 on 97 × 287 × 95 unknowns a component;
-// this kernel takes 48 and 61.  320 threads: with more, the registers of two blocks per SM do not hold the planes
-// ahead (352 threads: 70 µs); 24 rows: the halo of a nearly square tile is the smallest.
+// What bounds it: latency at 20 warps per SM (fixed-latency chains, the barrier of each plane, shared memory; its loads
+// wait no more, and it moves its compulsory bytes at 2.4 TB/s).  A block takes a tile of tj × tk columns (tj ≤ 24 rows of
+// the unit-stride axis; both split evenly), a column per thread, and marches over `chunk` planes i.  A thread reads its
+// own column (and one element of the tile's halo) straight into registers two planes ahead, forms P, and leaves it in
+// shared memory for its neighbours: three planes in turn, so that one barrier a plane suffices.  The plaquettes of plane
+// i − 1 that plane i needs are the thread's own, kept in registers.  Each plane is read once per tile with a halo of one
+// row and column.  The conductivities are a byte per link where they have at most 256 values (padding, materials), looked
+// up in shared memory.  One thread per node reading its 36 neighbours through L1 fetched each plane several times from L2,
+// and the direction was a pass of its own: 57 + 24 µs on the 256×128×32 ramp, 78 + 31 on 97 × 287 × 95 unknowns a
+// component; this kernel takes 48 and 61.  320 threads: with more, the registers of two blocks per SM do not hold the
+// planes ahead (352 threads: 70 µs); 24 rows: the halo of a nearly square tile is the smallest.
 struct ApplyArgs {
   const double *P[3];
   const void *Z[3];

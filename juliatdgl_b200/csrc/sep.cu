@@ -881,12 +881,13 @@ __device__ __forceinline__ void linesolve_staged_b(const Blk bk, T * const &Xh, 
   }
 }
 
-// The same solve with a line per warp and both components of a line together: a lane holds its chunk of CM right-hand sides and pivots in registers from the load to the
-// solution, so each is read from shared memory once, and the two components' recurrences, whose multipliers are the
-// same, run interleaved.  What bounds the staged kernel above is the latency of its chains (FP64 multiply and add
-// without contraction) at two blocks per SM; it took the components one after the other, and keeps FP64 right-hand
-// sides in shared memory.  The same operations in the same order: the same bits.  The ramp on 256×128×32 cells:
-// 39 → 33 µs per solve, 95 points of 287 × 95 lines 61 → 46.  Lines of more than 32 × LS3_MAX points take the staged kernel.
+// The same solve with a line per warp and both components of a line together: a lane holds its chunk of CM right-hand
+// sides and pivots in registers from the load to the solution, so each is read from shared memory once, and the two
+// components' recurrences, whose multipliers are the same, run interleaved.  What bounds the staged kernel above is the
+// latency of its chains (FP64 multiply and add without contraction) at two blocks per SM; it took the components one
+// after the other, and keeps FP64 right-hand sides in shared memory.  The same operations in the same order: the same
+// bits.  The ramp on 256×128×32 cells: 39 → 33 µs per solve, 95 points of 287 × 95 lines 61 → 46.  Lines of more than
+// 32 × LS3_MAX points take the staged kernel.
 const int LS3_MAX = 13;
 // the row of node i: LS2_ROW entries a node, and one more per chunk of an even length, so that the rows of consecutive
 // lanes are an odd number of entries apart (distinct banks)
@@ -1014,8 +1015,8 @@ __device__ __forceinline__ void linesolve_warp_b(const Blk bk, T * const &Xh, T 
         vy[u] = y;
         vz[u] = z;
       }
-    // X from Y and Z at the node and the next one (the chunk's last node: the next lane's first; the shuffles also
-    // order every lane's reads of X above before the writes here)
+    // X from Y and Z at the node and the next one (the chunk's last node: the next lane's first; a lane's
+    // solution depends on the X it read above, so its neighbour's write below, formed from it, comes after that read)
     double yn = __shfl_down_sync(0xffffffffu, vy[0], 1), zn = __shfl_down_sync(0xffffffffu, vz[0], 1);
 #pragma unroll
     for (int u = CM - 1; u >= 0; u--) {

@@ -20,13 +20,14 @@ namespace {
 // tile), k in index order (fma from 0).  Both axes, both directions and all components and classes (blk.z) of a
 // direction's product are one launch.
 //
-// What bounds it: FP32 multiply-adds.  A block takes bm outputs (⌈h / 64⌉ equal tiles, rounded to 8: 48 for h = 144,
-// 40 for 73) of HG_N = 128 points, 8 × 8 outputs a thread, so four 128-bit shared loads (six wavefronts a warp) feed
-// 64 multiply-adds; three stages of 16 k in flight by cp.async (40 KB a block, so that registers, not shared memory,
-// limit the blocks per SM).  The loads along k are element by element (class rows start at any column), so their places
-// are constants and their predicates one byte count: 96 µs for the row product of 95 planes of 287 × 95 points instead
-// of 111.  Before, each component and class had its own launch of 48 × 96 tiles without prefetching: 36 launches of
-// 25 µs per PCG iteration there, two blocks per SM each.
+// What bounds it: the operands' shared-memory loads and issue (43 to 58 % of the cycles issue, at 13 to 15 warps per
+// SM).  A block takes bm outputs (⌈h / 64⌉ equal tiles, rounded to 8: 48 for h = 144, 40 for 73) of HG_N = 128 points,
+// 8 × 8 outputs a thread, so four 128-bit shared loads (six wavefronts a warp) feed 64 multiply-adds; three stages of
+// 16 k in flight by cp.async (40 KB a block: registers and shared memory both leave five blocks of 96 threads per SM).
+// The loads along k are element by element (class rows start at any column), so their places are constants and their
+// predicates one byte count: 96 µs for the row product of 95 planes of 287 × 95 points instead of 111.  Before, each
+// component and class had its own launch of 48 × 96 tiles without prefetching: 36 launches of 25 µs per PCG iteration
+// there, two blocks per SM each.
 enum HMode { ROW_F, ROW_I, COL_F, COL_I };
 const int HG_N = 128, HG_K = 16, HG_ST = 3, HG_WS = 64, HG_DS = HG_N + 12;
 

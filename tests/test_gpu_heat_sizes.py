@@ -1,5 +1,5 @@
 """The heat model's sweep by planes at its edges: fewer columns than a warp, more than a block's threads, more than its
-shared memory holds, spacings whose squares are powers of two and not, one cell along an axis; device against the
+shared memory holds, spacings whose squares are powers of two and not, two cells along each axis; device against the
 oracle, Ψ and links at the exact-solve tolerance 1e-11, the temperature field too."""
 import numpy as np
 import pytest

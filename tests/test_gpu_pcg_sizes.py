@@ -1,5 +1,5 @@
-"""The PCG's A·p at the edges of its tiles (24 | 25 rows, 13 | 14 columns, a single cell along an axis, one plane and
-several per block), with conductivities of a few values (coded) and of more than 256 (as they are), each
+"""The PCG's A·p at the edges of its tiles along j (24 | 25 rows and more, a block of two cells along each axis; one plane
+per block and one tile along k), with conductivities of a few values (coded) and of more than 256 (as they are), each
 preconditioner; device against the oracle at the PCG's bar of 1e-7, the solves' iterations within one per step."""
 import numpy as np
 import pytest

@@ -1,6 +1,6 @@
 """The separable inverse at the edges of its transforms' tiles: extents where the components' row chunks differ in number
 or kind (48 | 49 and 96 | 97 rows), remainders of the register tiles, the smallest planes, and planes that take the batched products (several planes to a
-tile of points, both parities of each extent), lines of every chunk length (and too long for one warp); FP64 and FP32, against
+tile of points, both parities of each extent), lines of one to four nodes a lane and too long for one warp; FP64 and FP32, against
 the oracle's dense three-axis transforms at the tolerances of the parity test."""
 import numpy as np
 import pytest
